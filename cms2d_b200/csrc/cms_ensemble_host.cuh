@@ -11,7 +11,10 @@
 //
 // Layout: the launch's blocks (at most the device's resident capacity) are
 // split among the members in proportion to their unknowns, at least one
-// each; cms_ensemble_set_tiles picks the total (the autotuner in
+// each.  When every member's tiles fit one SM each, the blocks are those of
+// the resident form of the reduced solves (six 10k-cell inlets, one step:
+// 146 ms with the streaming form, 83 ms resident); cms_ensemble_set_tiles
+// picks the total (the autotuner in
 // cms2d_b200/ensemble.py times the candidates).
 #pragma once
 
@@ -24,6 +27,9 @@ struct cms_ensemble {
   std::vector<int> tiles;  // per member
   int total_tiles = 0;
   int batched = 0;  // 1: the solves run as batched persistent launches
+  bool resident = false;  // the tiles are those of the resident form
+  int res_nr = 0;         // its rows per thread and shared memory (largest member)
+  size_t res_smem = 0;
   cms::PersistArgs<float>* d_args = nullptr;
   cms::PersistArgs<float>* h_args = nullptr;  // pinned
   cms::SchurArgs* d_sargs = nullptr;           // reduced inner solves (every member in reduced form)
@@ -37,8 +43,54 @@ namespace cms {
 
 using Ens = ::cms_ensemble;
 
+// Splits at most total blocks (0: one per SM) among the members for the
+// resident form of the reduced solves (cms_resident.cuh) and builds their
+// tables; false when a member does not take it or its tiles do not fit.
+static bool ensemble_layout_resident(Ens* E, int total) {
+  const int M = (int)E->m.size();
+  size_t smem = 0;
+  const int blocks = resident_blocks(E->dev, &smem);
+  if (total <= 0) total = blocks;
+  if (total > blocks || total < M) return false;
+  double nsum = 0.0;
+  for (auto* F : E->m) {
+    if (!resident_wanted(F->S)) return false;
+    nsum += F->n - F->S->hp.gstart[1];
+  }
+  if (nsum > (double)total * RES_NRMAX * RES_BS) return false;
+  std::vector<int> t(M);
+  int used = 0;
+  for (int i = 0; i < M; ++i) {
+    Solver* S = E->m[i]->S;
+    const double nB = S->hp.n - S->hp.gstart[1];
+    t[i] = std::max(1, std::min((int)std::floor(total * nB / nsum), resident_count(S, total)));
+    used += t[i];
+  }
+  while (used > total) {
+    const int j = (int)(std::max_element(t.begin(), t.end()) - t.begin());
+    --t[j];
+    --used;
+  }
+  E->res_nr = 1;
+  E->res_smem = 0;
+  for (int i = 0; i < M; ++i) {
+    Solver* S = E->m[i]->S;
+    if (resident_tables(S, t[i]) != CMS_OK || S->rs_tiles != t[i]) return false;
+    E->res_nr = std::max(E->res_nr, S->rs_nr);
+    E->res_smem = std::max(E->res_smem, S->rs_smem);
+  }
+  if (cudaFuncSetAttribute(resident_kernel(E->res_nr, true), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)smem) != cudaSuccess)
+    return false;
+  E->tiles = t;
+  E->total_tiles = used;
+  return true;
+}
+
 // Splits total blocks among the members by unknowns and builds their tables.
 static int ensemble_layout(Ens* E, int total) {
+  E->resident = ensemble_layout_resident(E, total);
+  if (E->resident) return CMS_OK;
   const int M = (int)E->m.size();
   const int cap = persist_capacity(E->dev);
   if (cap <= 0) return CMS_UNSUPPORTED;
@@ -94,11 +146,18 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
   } reset{E, act};
   // the reduced inner form when every member's solver takes it (as each
   // member's own step does), else the two-phase or exact factor
-  bool schur = true;
-  for (int j = 0; j < A_ && schur; ++j) {
+  bool schur = true, resident = E->resident;
+  for (int j = 0; j < A_; ++j) {
     Solver* S = E->m[act[j]]->S;
-    schur = S->opts.inner_relax == 2 && S->opts.ordering == CMS_ORDER_MULTICOLOR &&
-            schur_pattern(S, E->tiles[act[j]]) == CMS_OK;
+    schur = schur && S->opts.inner_relax == 2 && S->opts.ordering == CMS_ORDER_MULTICOLOR;
+    // (a member's own step may have left it with tables for its own tiles)
+    resident = resident && schur && resident_wanted(S) && resident_tables(S, E->tiles[act[j]]) == CMS_OK &&
+               S->rs_tiles == E->tiles[act[j]];
+  }
+  for (int j = 0; j < A_ && !resident; ++j) {
+    Solver* S = E->m[act[j]]->S;
+    if (build_tiles(S, E->tiles[act[j]]) != E->tiles[act[j]]) return CMS_DEVICE_ERROR;
+    schur = schur && schur_neighbours(S, E->tiles[act[j]]) == CMS_OK;
   }
   // the single-reduction form when every member's layout option asks for it
   // and every member's pattern is symmetric (the launch is one kernel)
@@ -159,10 +218,12 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
       KLAUNCH(S, P_VEC, (double)n * 12,
               (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
       CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
-      CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * E->tiles[i] * kProgressStride, S->stream));
+      if (!resident)
+        CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * E->tiles[i] * kProgressStride, S->stream));
       refine_inner_limits(S->opts, R[j]);
       if (schur) E->h_sargs[c] = make_schur_args(S, E->tiles[i], R[j].imax, R[j].itol);
-      else E->h_args[c] = make_args<float>(S, S->A32, S->W32, E->tiles[i], R[j].imax, 2, R[j].itol, 1);
+      if (resident) CHK(resident_tags(S, R[j].imax, &E->h_sargs[c].tag0));
+      if (!schur) E->h_args[c] = make_args<float>(S, S->A32, S->W32, E->tiles[i], R[j].imax, 2, R[j].itol, 1);
       for (int t = 0; t < E->tiles[i]; ++t) E->h_bmap[blocks++] = make_int2(c, t);
       CMS_CUDA(cudaEventRecord(E->ev_m[i], S->stream));
       CMS_CUDA(cudaStreamWaitEvent(E->stream, E->ev_m[i], 0));
@@ -174,7 +235,11 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
       CMS_CUDA(cudaMemcpyAsync(E->d_args, E->h_args, cont.size() * sizeof(PersistArgs<float>),
                                cudaMemcpyHostToDevice, E->stream));
     CMS_CUDA(cudaMemcpyAsync(E->d_bmap, E->h_bmap, blocks * sizeof(int2), cudaMemcpyHostToDevice, E->stream));
-    if (schur) {
+    if (resident) {
+      void* kargs[] = {&E->d_sargs, &E->d_bmap};
+      CMS_CUDA(cudaLaunchCooperativeKernel(resident_kernel(E->res_nr, true), dim3(blocks), dim3(RES_BS), kargs,
+                                           E->res_smem, E->stream));
+    } else if (schur) {
       void* kargs[] = {&E->d_sargs, &E->d_bmap};
       // the layout the ensemble's tile split was sized for (256 threads per block)
       const void* kern = sr ? (const void*)k_schur_batched<TPB, 2, 1> : (const void*)k_schur_batched<TPB, 2, 0>;

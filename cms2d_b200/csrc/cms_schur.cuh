@@ -90,6 +90,18 @@ struct SchurArgs {
   int maxit;
   double tol;
   unsigned int spin_limit;
+  // resident form only (cms_resident.cuh): Chat's columns as indices into the
+  // tile's own and halo rows, rows other tiles gather, halo rows per tile,
+  // slot-pair offsets per 32-row slice, exchanged words, first tag of the launch
+  const unsigned short* lcol;  // [KC][nB]
+  const int* rexp;             // [nB] word of a row that other tiles gather (-1: none)
+  const int *tptr, *trow;      // [ntiles+1], the tiles' reduced rows
+  const int *hptr, *hrow;      // [ntiles+1], their halo rows' words
+  const int *slptr, *sloff;    // [ntiles], offsets of a tile's slices from its first
+  ulonglong2* xst;             // words (s, t), tag
+  unsigned long long* xnu;     // words nu, tag
+  ulonglong2* slots;           // [2][NSMAX][ntiles] sum, tag
+  unsigned int tag0;
 };
 
 // sinv: 1/d_r for group-0 rows, 1/s_r for B rows with

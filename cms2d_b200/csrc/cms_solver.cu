@@ -22,6 +22,7 @@
 #include "cms_legacy.cuh"
 #include "cms_order.h"
 #include "cms_persist.cuh"
+#include "cms_resident.cuh"
 #include "cms_schur.cuh"
 #include "cmsgpu.h"
 
@@ -102,6 +103,19 @@ struct cms_solver {
   float *d_scoff = nullptr, *d_ssinv = nullptr, *d_sst = nullptr;
   signed char* d_sccnt = nullptr;
   size_t cap_sdep = 0;
+  // its resident form (cms_resident.cuh): tiles of the tables (0 none) and of
+  // the last ones that did not fit, rows per thread, shared memory of the launch
+  int rs_tiles = 0, rs_unfit = 0, rs_nr = 0;
+  size_t rs_smem = 0;
+  unsigned short* d_rlcol = nullptr;
+  int* d_rexp = nullptr;
+  size_t rs_words = 0;  // exchanged words (capacity of d_rxst, d_rxnu)
+  int *d_rtptr = nullptr, *d_rtrow = nullptr, *d_rhptr = nullptr, *d_rslptr = nullptr, *d_rhrow = nullptr,
+      *d_rsloff = nullptr;
+  ulonglong2 *d_rxst = nullptr, *d_rslots = nullptr;
+  unsigned long long* d_rxnu = nullptr;
+  size_t cap_rhrow = 0, cap_rsloff = 0;
+  unsigned int rs_tag = 1;  // first tag not used by any launch so far
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   int cur_relax = 0;  // the FP32 factor in A32 is the two-phase one (k_ilu0_relax)
   int cur_fuse = 0;   // inner solves of refinement: update folded into the next iteration
@@ -773,11 +787,10 @@ static int resid64(Solver* S, Mat<TA>& A, const double* b, const TX* x, double* 
 
 // Pattern of the reduced inner system (cms_schur.cuh): Chat's columns per B
 // row (direct couplings to B rows and the B neighbours of each group-0
-// neighbour, the row itself excluded), once per handle; the neighbour-tile
-// lists under Chat for the persistent tiles, rebuilt when the tile count
-// changes.  CMS_UNSUPPORTED when the ordering has no independent first group
-// or a reduced row has more than KSC entries.
-static int schur_pattern(Solver* S, int tiles) {
+// neighbour, the row itself excluded), once per handle.  CMS_UNSUPPORTED when
+// the ordering has no independent first group or a reduced row has more than
+// KSC entries.
+static int schur_pattern(Solver* S) {
   const HostPattern& P = S->hp;
   const int n = P.n;
   if (S->sc_state < 0) return CMS_UNSUPPORTED;
@@ -855,14 +868,31 @@ static int schur_pattern(Solver* S, int tiles) {
     S->sc_tiles = 0;
     S->sc_state = 1;
   }
-  if (S->sc_tiles == tiles) return CMS_OK;
-  // neighbour tiles under Chat (tile t = natural cells [t n / nt, (t+1) n / nt))
-  const int g1 = P.gstart[1], nB = n - g1;
-  std::vector<int> ccol((size_t)S->sc_KC * nB);
-  std::vector<signed char> cnt(nB);
+  return CMS_OK;
+}
+
+// Chat's columns and counts back on the host, for tables that depend on tiles.
+static int schur_host_pattern(Solver* S, std::vector<int>& ccol, std::vector<signed char>& cnt) {
+  const size_t nB = S->hp.n - S->hp.gstart[1];
+  ccol.resize(S->sc_KC * nB);
+  cnt.resize(nB);
   CMS_CUDA(cudaMemcpyAsync(ccol.data(), S->d_sccol, ccol.size() * sizeof(int), cudaMemcpyDeviceToHost, S->stream));
   CMS_CUDA(cudaMemcpyAsync(cnt.data(), S->d_sccnt, cnt.size(), cudaMemcpyDeviceToHost, S->stream));
   CMS_CUDA(cudaStreamSynchronize(S->stream));
+  return CMS_OK;
+}
+
+// The neighbour-tile lists under Chat for the persistent tiles, rebuilt when
+// the tile count changes.
+static int schur_neighbours(Solver* S, int tiles) {
+  CHK(schur_pattern(S));
+  if (S->sc_tiles == tiles) return CMS_OK;
+  // neighbour tiles under Chat (tile t = natural cells [t n / nt, (t+1) n / nt))
+  const HostPattern& P = S->hp;
+  const int n = P.n, g1 = P.gstart[1], nB = n - g1;
+  std::vector<int> ccol;
+  std::vector<signed char> cnt;
+  CHK(schur_host_pattern(S, ccol, cnt));
   std::vector<int> tstart(tiles + 1);
   for (int t = 0; t <= tiles; ++t) tstart[t] = (int)((long long)t * n / tiles);
   std::vector<int> tile_nat(n);
@@ -896,6 +926,225 @@ static int schur_pattern(Solver* S, int tiles) {
                              S->stream));
   CMS_CUDA(cudaStreamSynchronize(S->stream));
   S->sc_tiles = tiles;
+  return CMS_OK;
+}
+
+// Blocks of the resident kernel the device can hold at once (one per SM) and
+// the dynamic shared memory each may use; 0 when it cannot be launched.
+static int resident_blocks(int dev, size_t* smem) {
+  int coop = 0, nsm = 0, optin = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  size_t most = (size_t)optin;
+  for (int nr = 1; nr <= RES_NRMAX; nr *= 2) {
+    for (int b = 0; b < 2; ++b) {
+      cudaFuncAttributes fa;
+      if (cudaFuncGetAttributes(&fa, resident_kernel(nr, b != 0)) != cudaSuccess || fa.sharedSizeBytes >= (size_t)optin) {
+        cudaGetLastError();
+        return 0;
+      }
+      most = std::min(most, (size_t)optin - fa.sharedSizeBytes);
+    }
+  }
+  *smem = most;
+  return std::min(nsm, GRID_CAP);
+}
+
+// Tiles of the resident form: nt sets of B rows of (nearly) equal size, as
+// square as the numbering allows, so that few rows are gathered by another
+// tile: strips of consecutive natural cells about as high as a tile, each cut
+// along the breadth-first order from its first cell.  (With whole strips per
+// tile, 6.8 grid rows of the 1M-cell system, 2000-2800 of a tile's 3400 rows
+// were halo rows; square tiles have about 350.)  The grid's width in cells is
+// the median natural-number distance from a cell to its farthest-numbered
+// neighbour (the cell north of it).
+static void resident_partition(const HostPattern& P, int nt, std::vector<int>& tile_of) {
+  const int n = P.n, g1 = P.gstart[1], nB = n - g1;
+  auto for_neighbours = [&](int r, auto&& f) {
+    for (int s = 0; s < P.nlo[r]; ++s) f(P.col[(size_t)s * n + r]);
+    for (int s = 0; s < P.nup[r]; ++s) f(P.col[(size_t)(P.KL + s) * n + r]);
+  };
+  tile_of.assign(nB, 0);
+  std::vector<int> jump;
+  for (int c = 0; c < n; c += std::max(1, n / 4096)) {
+    int m = 0;
+    for_neighbours(P.iperm[c], [&](int k) { m = std::max(m, P.perm[k] - c); });
+    if (m > 0) jump.push_back(m);
+  }
+  int width = 1;
+  if (!jump.empty()) {
+    std::nth_element(jump.begin(), jump.begin() + jump.size() / 2, jump.end());
+    width = jump[jump.size() / 2];
+  }
+  const double side = std::sqrt((double)n / nt);
+  const int per = std::max(1, std::min(nt, (int)(width / side + 0.5)));  // tiles per strip
+  const int strips = (nt + per - 1) / per;
+  std::vector<char> seen(n, 0);  // by natural number
+  std::vector<int> queue;
+  long long done = 0;  // B rows of the strips so far
+  int c0 = 0;
+  for (int s = 0; s < strips; ++s) {
+    const int t0 = (int)((long long)s * nt / strips), t1 = (int)((long long)(s + 1) * nt / strips);
+    const long long want = (long long)nB * t1 / nt;
+    int c1 = c0;
+    long long rows = done;
+    while (c1 < n && (rows < want || s == strips - 1)) rows += P.iperm[c1++] >= g1;
+    const long long mine = rows - done;
+    long long k = 0;
+    for (int c = c0; c < c1; ++c) {  // (a strip in several pieces: one after the other)
+      if (seen[c]) continue;
+      queue.assign(1, c);
+      seen[c] = 1;
+      for (size_t h = 0; h < queue.size(); ++h) {
+        const int r = P.iperm[queue[h]];
+        if (r >= g1) {
+          tile_of[r - g1] = t0 + (int)std::min<long long>(k * (t1 - t0) / std::max(mine, 1ll), t1 - t0 - 1);
+          ++k;
+        }
+        for_neighbours(r, [&](int j) {
+          const int cj = P.perm[j];
+          if (cj >= c0 && cj < c1 && !seen[cj]) {
+            seen[cj] = 1;
+            queue.push_back(cj);
+          }
+        });
+      }
+    }
+    done = rows;
+    c0 = c1;
+  }
+}
+
+// Tables of the resident form for a number of tiles: a tile's rows, the index
+// of each of Chat's columns among its tile's own and halo rows, the halo rows,
+// the rows other tiles gather and the slices' slot pairs.  rs_tiles = 0 when
+// a tile has too many rows or needs more shared memory than an SM has.
+static int resident_tables(Solver* S, int tiles) {
+  if (S->rs_tiles == tiles) return CMS_OK;
+  S->rs_tiles = 0;
+  if (S->rs_unfit == tiles) return CMS_OK;
+  S->rs_unfit = tiles;
+  CHK(schur_pattern(S));
+  const HostPattern& P = S->hp;
+  const int g1 = P.gstart[1], nB = P.n - g1, KC = S->sc_KC;
+  size_t limit = 0;
+  if (!S->sc_sym || tiles > resident_blocks(S->dev, &limit) || nB > (long long)tiles * RES_NRMAX * RES_BS)
+    return CMS_OK;
+  std::vector<int> ccol, tile_of, loc(nB), nb(tiles, 0), tptr(tiles + 1, 0), trow(nB);
+  std::vector<signed char> cnt;
+  CHK(schur_host_pattern(S, ccol, cnt));
+  resident_partition(P, tiles, tile_of);
+  for (int i = 0; i < nB; ++i) loc[i] = nb[tile_of[i]]++;
+  const int most = *std::max_element(nb.begin(), nb.end());
+  if (most > RES_NRMAX * RES_BS) return CMS_OK;
+  for (int t = 0; t < tiles; ++t) tptr[t + 1] = tptr[t] + nb[t];
+  for (int i = 0; i < nB; ++i) trow[tptr[tile_of[i]] + loc[i]] = i;
+  std::vector<std::vector<int>> halo(tiles);
+  std::vector<int> exported(nB, -1);  // the row's word
+  for (int i = 0; i < nB; ++i)
+    for (int q = 0; q < cnt[i]; ++q) {
+      const int c = ccol[(size_t)q * nB + i] - g1;
+      if (tile_of[c] != tile_of[i]) {
+        halo[tile_of[i]].push_back(c);
+        exported[c] = 0;
+      }
+    }
+  std::vector<int> hptr(tiles + 1, 0), hrow, slptr(tiles), sloff;
+  for (int t = 0; t < tiles; ++t) {
+    std::sort(halo[t].begin(), halo[t].end());
+    halo[t].erase(std::unique(halo[t].begin(), halo[t].end()), halo[t].end());
+    hrow.insert(hrow.end(), halo[t].begin(), halo[t].end());
+    hptr[t + 1] = (int)hrow.size();
+  }
+  // words: a tile's are consecutive and start on a 128-byte line of their own
+  // (two tiles' words in one line slow both the stores and the polls)
+  size_t words = 0;
+  for (int t = 0; t < tiles; ++t) {
+    words = (words + 15) / 16 * 16;
+    for (int k = tptr[t]; k < tptr[t + 1]; ++k)
+      if (exported[trow[k]] >= 0) exported[trow[k]] = (int)words++;
+  }
+  std::vector<int> hword(hrow.size());
+  for (size_t k = 0; k < hrow.size(); ++k) hword[k] = exported[hrow[k]];
+  // slot pairs per slice: half the largest count of its 32 rows, rounded up
+  std::vector<std::vector<int>> width(tiles);
+  for (int t = 0; t < tiles; ++t) width[t].assign((nb[t] + 31) / 32, 0);
+  for (int i = 0; i < nB; ++i) {
+    int& w = width[tile_of[i]][loc[i] / 32];
+    w = std::max(w, (cnt[i] + 1) / 2);
+  }
+  size_t smem = 0;
+  for (int t = 0; t < tiles; ++t) {
+    slptr[t] = (int)sloff.size();
+    int o = 0;
+    for (int w : width[t]) {
+      sloff.push_back(o);
+      o += w;
+    }
+    sloff.push_back(o);
+    const int nh = hptr[t + 1] - hptr[t];
+    if (nb[t] + 31 + nh > 65535) return CMS_OK;
+    smem = std::max(smem, resident_smem(o, nb[t], nh));
+  }
+  if (smem > limit) return CMS_OK;
+  std::vector<unsigned short> lcol((size_t)KC * nB);
+  for (int i = 0; i < nB; ++i) {
+    const std::vector<int>& H = halo[tile_of[i]];
+    for (int q = 0; q < KC; ++q) {
+      const int c = ccol[(size_t)q * nB + i] - g1;
+      lcol[(size_t)q * nB + i] =
+          (unsigned short)(tile_of[c] == tile_of[i]
+                               ? loc[c]
+                               : (nb[tile_of[i]] + 31) / 32 * 32 + (int)(std::lower_bound(H.begin(), H.end(), c) - H.begin()));
+    }
+  }
+  if (!S->d_rlcol) {
+    CHK(S->alloc(&S->d_rlcol, lcol.size()));
+    CHK(S->alloc(&S->d_rexp, (size_t)nB));
+    CHK(S->alloc(&S->d_rtrow, (size_t)nB));
+    CHK(S->alloc(&S->d_rtptr, (size_t)GRID_CAP + 1));
+    CHK(S->alloc(&S->d_rhptr, (size_t)GRID_CAP + 1));
+    CHK(S->alloc(&S->d_rslptr, (size_t)GRID_CAP));
+    CHK(S->alloc(&S->d_rslots, (size_t)2 * (NSMAX * GRID_CAP + RES_TOT)));
+  }
+  if (words + 1 > S->rs_words) {
+    CHK(S->alloc(&S->d_rxst, words + 1));
+    CHK(S->alloc(&S->d_rxnu, words + 1));
+    S->rs_words = words + 1;
+  }
+  if (hrow.size() + 1 > S->cap_rhrow) {
+    CHK(S->alloc(&S->d_rhrow, hrow.size() + 1));
+    S->cap_rhrow = hrow.size() + 1;
+  }
+  if (sloff.size() > S->cap_rsloff) {
+    CHK(S->alloc(&S->d_rsloff, sloff.size()));
+    S->cap_rsloff = sloff.size();
+  }
+  cudaStream_t s = S->stream;
+  auto up = [&](void* d, const void* h, size_t nbytes) {
+    return nbytes == 0 ? cudaSuccess : cudaMemcpyAsync(d, h, nbytes, cudaMemcpyHostToDevice, s);
+  };
+  CMS_CUDA(up(S->d_rlcol, lcol.data(), lcol.size() * sizeof(unsigned short)));
+  CMS_CUDA(up(S->d_rexp, exported.data(), exported.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rtrow, trow.data(), trow.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rtptr, tptr.data(), tptr.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rhptr, hptr.data(), hptr.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rhrow, hword.data(), hword.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rslptr, slptr.data(), slptr.size() * sizeof(int)));
+  CMS_CUDA(up(S->d_rsloff, sloff.data(), sloff.size() * sizeof(int)));
+  CMS_CUDA(cudaStreamSynchronize(s));
+  int nr = 1;
+  while (most > nr * RES_BS) nr *= 2;
+  for (int b = 0; b < 2; ++b)
+    CMS_CUDA(cudaFuncSetAttribute(resident_kernel(nr, b != 0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  S->rs_smem = smem;
+  S->rs_nr = nr;
+  S->rs_tiles = tiles;
+  S->rs_unfit = 0;
   return CMS_OK;
 }
 
@@ -955,7 +1204,52 @@ static SchurArgs make_schur_args(Solver* S, int tiles, int maxit, double tol) {
   a.yb = S->W32.vv[4];
   a.part = S->d_ppart; a.bar = &S->d_st->bar; a.st = S->d_st;
   a.maxit = maxit; a.tol = tol; a.spin_limit = kSpinLimit;
+  if (S->rs_tiles > 0) {
+    a.lcol = S->d_rlcol; a.rexp = S->d_rexp; a.tptr = S->d_rtptr; a.trow = S->d_rtrow;
+    a.hptr = S->d_rhptr; a.hrow = S->d_rhrow; a.slptr = S->d_rslptr; a.sloff = S->d_rsloff;
+    a.xst = S->d_rxst; a.xnu = S->d_rxnu; a.slots = S->d_rslots;
+  }
   return a;
+}
+
+// Tags of a resident launch of at most maxit iterations; the words are
+// cleared before the 32-bit tags would run over.
+static int resident_tags(Solver* S, int maxit, unsigned int* tag0) {
+  const unsigned int need = (unsigned int)std::max(maxit, 0) + 2u;
+  if (S->rs_tag > 0xffffffffu - need) {
+    CMS_CUDA(cudaMemsetAsync(S->d_rxst, 0, S->rs_words * sizeof(ulonglong2), S->stream));
+    CMS_CUDA(cudaMemsetAsync(S->d_rxnu, 0, S->rs_words * sizeof(unsigned long long), S->stream));
+    CMS_CUDA(cudaMemsetAsync(S->d_rslots, 0, (size_t)2 * (NSMAX * GRID_CAP + RES_TOT) * sizeof(ulonglong2), S->stream));
+    S->rs_tag = 1;
+  }
+  *tag0 = S->rs_tag;
+  S->rs_tag += need;
+  return CMS_OK;
+}
+
+// Tiles of the resident form: one per SM, at least kResRows rows each (a
+// 30k-cell inlet-like system: 4.6 us per iteration with 128 rows, 5.2 with 256,
+// 5.3 with 512; fewer rows leave warps idle and add blocks to the sums).
+constexpr int kResRows = 128;
+static int resident_count(const Solver* S, int blocks) {
+  const int nB = S->hp.n - S->hp.gstart[1];
+  return std::max(1, std::min(blocks, (nB + kResRows - 1) / kResRows));
+}
+
+// The automatic layout of the reduced inner solve on a multicolour ordering:
+// the resident form where the system fits it.
+static bool resident_wanted(const Solver* S) {
+  const int lay = S->opts.reduced_layout;
+  return !(lay >= 1 && lay <= kSchurLayouts) && S->opts.inner_relax == 2 &&
+         S->opts.ordering == CMS_ORDER_MULTICOLOR && S->hp.G >= 2;
+}
+
+// Whether the resident form runs; builds its tables when it does.
+static bool resident_choose(Solver* S) {
+  if (!resident_wanted(S)) return false;
+  size_t smem = 0;
+  const int blocks = resident_blocks(S->dev, &smem);
+  return blocks > 0 && resident_tables(S, resident_count(S, blocks)) == CMS_OK && S->rs_tiles > 0;
 }
 
 // Layout of the reduced kernel for this handle (cms_solver_opts.reduced_layout,
@@ -991,14 +1285,21 @@ static int schur_tiles(Solver* S, int layout) {
 }
 
 // The reduced FP32 inner solve (W32.b -> W32.x) as one cooperative launch.
-static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol) {
+static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, bool resident) {
+  if (resident) tiles = S->rs_tiles;
   SchurArgs a = make_schur_args(S, tiles, maxit, tol);
   const SchurLayout L = schur_layout(schur_layout_run(S));
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
-  CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
+  if (resident)
+    CHK(resident_tags(S, maxit, &a.tag0));
+  else
+    CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
   void* args[] = {&a};
   prof_begin(S);
-  const cudaError_t e = cudaLaunchCooperativeKernel(L.single, dim3(tiles), dim3(L.bs), args, 0, S->stream);
+  const cudaError_t e =
+      resident ? cudaLaunchCooperativeKernel(resident_kernel(S->rs_nr, false), dim3(tiles), dim3(RES_BS), args,
+                                             S->rs_smem, S->stream)
+               : cudaLaunchCooperativeKernel(L.single, dim3(tiles), dim3(L.bs), args, 0, S->stream);
   if (e != cudaSuccess) {
     std::snprintf(g_last_error, sizeof(g_last_error), "cooperative launch (reduced BiCGStab): %s",
                   cudaGetErrorString(e));
@@ -1138,9 +1439,10 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
   const bool mc_persist = nsolv == 3 && S->opts.ordering == CMS_ORDER_MULTICOLOR && !S->opts.multi_kernel &&
                           persist_tiles(S) > 0;
   bool schur = mc_persist && S->opts.inner_relax == 2;
-  if (schur) {  // the tiles of the reduced kernel's layout
+  const bool resident = schur && resident_choose(S);
+  if (schur && !resident) {  // the tiles of the reduced kernel's layout
     const int nt = schur_tiles(S, schur_layout_index(S));
-    schur = nt > 0 && build_tiles(S, nt) == nt && schur_pattern(S, S->ptiles) == CMS_OK;
+    schur = nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->ptiles) == CMS_OK;
   }
   const bool relax = !schur && mc_persist && S->opts.inner_relax && P.G > 2;
   struct RelaxScope {  // the flags describe A32's factor and its solves only while this solve runs
@@ -1176,7 +1478,7 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
     refine_inner_limits(S->opts, R);
     KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
     if (schur) {
-      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol));  // tiles built above for its layout
+      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, resident));  // tiles built above for its layout
     } else if (nsolv == 3) {
       CHK(run_bicgstab<float>(S, S->A32, S->W32, R.imax, 2, R.itol, 1, false));
     } else {
