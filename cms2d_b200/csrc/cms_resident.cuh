@@ -2,25 +2,32 @@
 //
 // The single-reduction iteration of cms_schur.cuh (schur_body_sr: the same
 // recurrences and the same arithmetic per row), for systems whose tiles fit
-// one SM each.  In the streaming form an iteration of the 1M-cell system
-// took 28 us although its 100 MB stay in L2: two gather phases of 9 us of
-// dependent L1/L2 loads (each acquire empties L1) and 9 us of fences,
-// progress flags, arrival counter and partial sums.  Here
+// one SM each.  In the streaming form an iteration takes 14-16 us on small
+// systems and 28 us on the 1M-cell one although its 100 MB stay in L2: gather
+// phases of dependent L1/L2 loads (each acquire empties L1) and fences,
+// progress flags, an arrival counter and partial sums.  Here
 //
 //  * Chat's coefficients and columns stay in the block's shared memory for
 //    the whole launch (sliced ELL over 32-row slices, column = 16-bit index
-//    into the block's own and halo rows), and a thread keeps all nine vectors
-//    of its rows in registers; a gather reads shared memory only;
-//  * only rows that another tile gathers are written to global memory, each
+//    into the block's own and halo rows), and a thread keeps the vectors of
+//    its rows in registers; a gather reads shared memory only;
+//  * tiles are as square as the numbering allows (resident_partition), and
+//    only rows that another tile gathers are written to global memory, each
 //    as one word that holds the value and the iteration's tag (8 bytes for
 //    nu, 16 for s and t); a reader polls the word itself until the tag is the
-//    one it needs.  No fence, no progress flag and no L1 invalidation: a halo
-//    exchange costs one store and one load through L2;
-//  * the nine sums travel the same way: a block stores each of its partial
-//    sums with the tag, every block polls all blocks' words and adds them in
-//    the same fixed order, which is the grid barrier as well;
-//  * one warp forms the scalars of the recurrence (five FP64 divisions) while
-//    the others wait, instead of 32 warps forming them at once.
+//    one it needs.  No fence, no progress flag and no L1 invalidation: an
+//    exchange takes 550 cycles within a die and 950 across (measured; with
+//    release and acquire 1000 and 1600);
+//  * the nine sums travel the same way through one collecting tile, which is
+//    the grid barrier as well;
+//  * one warp forms the scalars of the recurrence while the others gather.
+//
+// Measured (one B200, kernel time per iteration, start and end of the launch
+// included, streaming form / this form): 1k cells 14.8 / 4.4 us, 30k 16.3 /
+// 4.6, 250k 16.9 / 6.4, 1M 28.8 / 15.0.  What bounds it: at 1M cells the
+// shared-memory wavefronts of the two gathers (about 3000 cycles of 4400
+// each); at 30k cells the three exchanges through L2 (about 5000 of 8300
+// cycles).
 //
 // Why a word is never overwritten too early.  nu of iteration i is replaced
 // in iteration i+1 after the sums of i, which a reader contributes to after
