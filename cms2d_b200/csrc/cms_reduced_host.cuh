@@ -1,0 +1,393 @@
+// Host side of the reduced Krylov solves (cms_reduced.cuh): tables per handle,
+// C's values per solve, the launches.  Included by cms_solver.cu after the
+// reduced system's pattern (schur_pattern) and the tiles (resident_partition).
+#pragma once
+
+namespace cms {
+
+// Shared memory of a tile besides its vectors and packed coefficients.
+template <typename T>
+static size_t red_smem_base(const RedTables& R, int t) {
+  const size_t hb = R.hb[t], ns = hb / 32, nsp = R.h_nsp[t], ne = R.h_ne[t], nos = R.h_nos[t];
+  auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
+  return up(sizeof(T) * (hb + R.h_nh[t])) + up(4 * (ns + 1)) + up(2 * hb) + up(8 * (nsp + 1)) + up(sizeof(T) * nsp) +
+         up(sizeof(T) * ne) + up(2 * ne) + up(2 * nos) + up(sizeof(T) * nos) + up(sizeof(T) * 3 * nos);
+}
+
+// How a launch with nvec vectors lays out its shared memory: the number of
+// vectors kept there (the last ones, the most used), then C's packed slices if
+// they fit too.  False when not even the gathered vector fits.
+template <typename T>
+static bool red_plan(const RedTables& R, int nvec, size_t limit, int* nvs, int* mat, size_t* smem) {
+  auto up = [](size_t b) { return (b + 15) & ~(size_t)15; };
+  auto need = [&](int v, int m) {
+    size_t most = 0;
+    for (int t = 0; t < R.tiles; ++t)
+      most = std::max(most, red_smem_base<T>(R, t) + v * up(sizeof(T) * R.hb[t]) +
+                                (m ? up(sizeof(T) * 64 * (size_t)R.h_npair[t]) + up(128 * (size_t)R.h_npair[t]) : 0));
+    return most;
+  };
+  int v = nvec;
+  while (v > 0 && need(v, 0) > limit) --v;
+  if (need(v, 0) > limit) return false;
+  *nvs = v;
+  *mat = v == nvec && need(v, 1) <= limit ? 1 : 0;
+  *smem = need(v, *mat);
+  return true;
+}
+
+// Dynamic shared memory the kernels may use, set as their attribute.
+static int red_limit(Solver* S, size_t* limit) {
+  int optin = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S->dev) != cudaSuccess) return CMS_DEVICE_ERROR;
+  const void* k[3] = {(const void*)k_red_bicg<double>, (const void*)k_red_gmres<double>,
+                      (const void*)k_red_gmres<float>};
+  size_t most = (size_t)optin;
+  for (const void* f : k) {
+    cudaFuncAttributes fa;
+    CMS_CUDA(cudaFuncGetAttributes(&fa, f));
+    if (fa.sharedSizeBytes >= (size_t)optin) return CMS_UNSUPPORTED;
+    most = std::min(most, (size_t)optin - fa.sharedSizeBytes);
+  }
+  for (const void* f : k) CMS_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  *limit = most;
+  return CMS_OK;
+}
+
+// Tables of the reduced Krylov solves for the handle's pattern, built on first
+// use.  S->rd.state: 1 built, -1 the pattern or its size does not take them.
+static int red_tables(Solver* S) {
+  RedTables& R = S->rd;
+  if (R.state != 0) return CMS_OK;
+  R.state = -1;
+  const HostPattern& P = S->hp;
+  if (P.G < 2 || P.G > GFLAT || schur_pattern(S) != CMS_OK || !S->sc_sym) return CMS_OK;
+  size_t rs_limit = 0;
+  const int blocks = resident_blocks(S->dev, &rs_limit);
+  if (blocks <= 0) return CMS_OK;
+  const int n = P.n, g1 = P.gstart[1], nB = n - g1, KC = S->sc_KC, G = P.G;
+  const int nt = resident_count(S, blocks);
+  if ((size_t)KC * nB > (size_t)INT32_MAX || (size_t)S->K * n > (size_t)INT32_MAX) return CMS_OK;
+  std::vector<int> ccol, tile_of, loc(nB), nb(nt, 0), tptr(nt + 1, 0), trow(nB), ttile(nB);
+  std::vector<signed char> cnt;
+  CHK(schur_host_pattern(S, ccol, cnt));
+  resident_partition(P, nt, tile_of);
+  for (int i = 0; i < nB; ++i) loc[i] = nb[tile_of[i]]++;
+  for (int t = 0; t < nt; ++t) tptr[t + 1] = tptr[t] + nb[t];
+  for (int i = 0; i < nB; ++i) {
+    trow[tptr[tile_of[i]] + loc[i]] = i;
+    ttile[tptr[tile_of[i]] + loc[i]] = tile_of[i];
+  }
+  // couplings among B rows (special rows), by side
+  auto lower = [&](int i, auto&& f) {
+    const int r = g1 + i;
+    for (int s = 0; s < P.nlo[r]; ++s) {
+      const size_t e = (size_t)s * n + r;
+      if (P.col[e] >= g1) f(P.col[e] - g1, (int)e);
+    }
+  };
+  auto upper = [&](int i, auto&& f) {
+    const int r = g1 + i;
+    for (int s = 0; s < P.nup[r]; ++s) {
+      const size_t e = (size_t)(P.KL + s) * n + r;
+      f(P.col[e] - g1, (int)e);
+    }
+  };
+  std::vector<char> special(nB, 0);
+  for (int i = 0; i < nB; ++i) {
+    bool sp = false;
+    lower(i, [&](int, int) { sp = true; });
+    upper(i, [&](int, int) { sp = true; });
+    special[i] = sp;
+  }
+  std::vector<int> group(nB);
+  for (int g = 1; g < G; ++g)
+    for (int r = P.gstart[g]; r < P.gstart[g + 1]; ++r) group[r - g1] = g;
+  // per tile: rows whose z (bit 2) or y (bit 1) it needs
+  const int nphase = (G - 2) + (G - 1);
+  std::vector<std::vector<int>> halo(nt);
+  std::vector<int> word(nB, -1);
+  std::vector<int> spp((size_t)nt * (nphase + 1)), spe, spoff, osptr(nt + 1, 0), osrow;
+  std::vector<int2> sprow;
+  std::vector<unsigned short> spcol, kind(nB, RED_SIMPLE);
+  std::vector<int> hptr(nt + 1, 0), hrow, slptr(nt), sloff, mbase(nt), tpad(nt);
+  std::vector<unsigned char> mark(nB, 0);
+  std::vector<int> lidx(nB, -1);
+  R.hb.assign(nt, 0);
+  R.h_nh.assign(nt, 0);
+  R.h_nsp.assign(nt, 0);
+  R.h_ne.assign(nt, 0);
+  R.h_nos.assign(nt, 0);
+  R.h_npair.assign(nt, 0);
+  std::vector<ushort2> plcol;
+  std::vector<int> touched, stack;
+  int pairs = 0, pad = 0;
+  for (int t = 0; t < nt; ++t) {
+    const int hb = (nb[t] + 31) / 32 * 32;
+    R.hb[t] = hb;
+    tpad[t] = pad;
+    pad += hb;
+    touched.clear();
+    auto need = [&](int i, int bits) {
+      if ((mark[i] & bits) == bits) return;
+      if (!mark[i]) touched.push_back(i);
+      mark[i] |= bits;
+      if (special[i]) stack.push_back(i);
+    };
+    auto drain = [&] {
+      while (!stack.empty()) {
+        const int i = stack.back();
+        stack.pop_back();
+        lower(i, [&](int j, int) { need(j, 1); });
+        if (mark[i] & 2) upper(i, [&](int j, int) { need(j, 3); });
+      }
+    };
+    for (int k = 0; k < nb[t]; ++k) need(trow[tptr[t] + k], 3);
+    for (int k = 0; k < nb[t]; ++k) {
+      const int i = trow[tptr[t] + k];
+      for (int q = 0; q < cnt[i]; ++q) need(ccol[(size_t)q * nB + i] - g1, 3);
+    }
+    drain();
+    for (int i : touched)
+      if (tile_of[i] != t) halo[t].push_back(i);
+    std::sort(halo[t].begin(), halo[t].end());
+    for (int k = 0; k < nb[t]; ++k) lidx[trow[tptr[t] + k]] = k;
+    for (size_t h = 0; h < halo[t].size(); ++h) {
+      lidx[halo[t][h]] = hb + (int)h;
+      word[halo[t][h]] = 0;
+    }
+    hrow.insert(hrow.end(), halo[t].begin(), halo[t].end());
+    hptr[t + 1] = (int)hrow.size();
+    R.h_nh[t] = (int)halo[t].size();
+    if (hb + R.h_nh[t] > 65535) return CMS_OK;
+    // special rows by phase
+    std::vector<int> sp;
+    for (int i : touched)
+      if (special[i]) sp.push_back(i);
+    std::sort(sp.begin(), sp.end());
+    const int s_first = (int)sprow.size(), e_first = (int)spoff.size();
+    int ph = 0;
+    auto phase = [&](int g, bool fwd) {
+      spp[(size_t)t * (nphase + 1) + ph++] = (int)sprow.size();
+      for (int i : sp) {
+        if (group[i] != g || (!fwd && !(mark[i] & 2))) continue;
+        sprow.push_back(make_int2(lidx[i], g1 + i));
+        spe.push_back((int)spoff.size());
+        auto entry = [&](int j, int e) {
+          spoff.push_back(e);
+          spcol.push_back((unsigned short)lidx[j]);
+        };
+        if (fwd) lower(i, entry);
+        else upper(i, entry);
+      }
+    };
+    for (int g = 2; g < G; ++g) phase(g, true);
+    for (int g = G - 1; g >= 1; --g) phase(g, false);
+    spp[(size_t)t * (nphase + 1) + ph] = (int)sprow.size();
+    R.h_nsp[t] = (int)sprow.size() - s_first;
+    R.h_ne[t] = (int)spoff.size() - e_first;
+    for (int k = 0; k < nb[t]; ++k) {
+      const int i = trow[tptr[t] + k];
+      if (!special[i]) continue;
+      kind[tptr[t] + k] = (unsigned short)R.h_nos[t]++;
+      osrow.push_back(k);
+    }
+    osptr[t + 1] = (int)osrow.size();
+    if (R.h_nos[t] >= RED_SIMPLE) return CMS_OK;
+    // slices: slot pairs per 32 rows, local columns in the packed order
+    slptr[t] = (int)sloff.size();
+    mbase[t] = pairs;
+    int o = 0;
+    for (int j = 0; j < hb / 32; ++j) {
+      int w = 0;
+      for (int k = j * 32; k < std::min(nb[t], j * 32 + 32); ++k) w = std::max(w, (cnt[trow[tptr[t] + k]] + 1) / 2);
+      sloff.push_back(o);
+      const size_t base = plcol.size();
+      plcol.resize(base + (size_t)w * 32);
+      for (int l = 0; l < 32; ++l) {
+        const int k = j * 32 + l, i = k < nb[t] ? trow[tptr[t] + k] : -1;
+        const unsigned short own = (unsigned short)std::min(k, nb[t] - 1);
+        for (int q = 0; q < w; ++q) {
+          auto lc = [&](int s) {
+            return i >= 0 && s < cnt[i] ? (unsigned short)lidx[ccol[(size_t)s * nB + i] - g1] : own;
+          };
+          plcol[base + (size_t)q * 32 + l] = make_ushort2(lc(2 * q), lc(2 * q + 1));
+        }
+      }
+      o += w;
+    }
+    sloff.push_back(o);
+    pairs += o;
+    R.h_npair[t] = o;
+    for (int i : touched) mark[i] = 0;
+  }
+  spe.push_back((int)spoff.size());
+  R.tiles = nt;
+  size_t limit = 0, smem = 0;
+  CHK(red_limit(S, &limit));
+  int nvs, mat;
+  if (!red_plan<double>(R, RED_NV_BICG, limit, &nvs, &mat, &smem)) return CMS_OK;
+  // words: a tile's are consecutive, on lines of their own
+  size_t words = 0;
+  std::vector<int> rexp(nB, -1);
+  for (int t = 0; t < nt; ++t) {
+    words = (words + 15) / 16 * 16;
+    for (int k = tptr[t]; k < tptr[t + 1]; ++k)
+      if (word[trow[k]] >= 0) rexp[k] = word[trow[k]] = (int)words++;
+  }
+  std::vector<int> hword(hrow.size());
+  for (size_t k = 0; k < hrow.size(); ++k) hword[k] = word[hrow[k]];
+  cudaStream_t s = S->stream;
+  auto put = [&](auto** d, const auto& h) -> int {
+    CHK(S->alloc(d, h.size()));
+    if (!h.empty()) CMS_CUDA(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, s));
+    return CMS_OK;
+  };
+  CHK(put(&R.tptr, tptr));
+  CHK(put(&R.trow, trow));
+  CHK(put(&R.ttile, ttile));
+  CHK(put(&R.tpad, tpad));
+  CHK(put(&R.rexp, rexp));
+  CHK(put(&R.kind, kind));
+  CHK(put(&R.hptr, hptr));
+  CHK(put(&R.hword, hword));
+  CHK(put(&R.slptr, slptr));
+  CHK(put(&R.sloff, sloff));
+  CHK(put(&R.mbase, mbase));
+  CHK(put(&R.plcol, plcol));
+  CHK(put(&R.spp, spp));
+  CHK(put(&R.sprow, sprow));
+  CHK(put(&R.spe, spe));
+  CHK(put(&R.spoff, spoff));
+  CHK(put(&R.spcol, spcol));
+  CHK(put(&R.osptr, osptr));
+  CHK(put(&R.osrow, osrow));
+  CHK(S->alloc(&R.xw, words + 1));
+  CHK(S->alloc(&R.slots, (size_t)2 * (NSMAX * nt + RES_TOT)));
+  CMS_CUDA(cudaStreamSynchronize(s));
+  R.words = words;
+  R.npad = pad;
+  R.pairs = pairs;
+  R.nphase = nphase;
+  R.nfwd = G - 2;
+  R.limit = limit;
+  R.state = 1;
+  return CMS_OK;
+}
+
+template <typename T>
+static RedBuf& red_buf(Solver* S) {
+  return sizeof(T) == 8 ? S->rd64 : S->rd32;
+}
+
+// Whether a solve runs in reduced form: a multicolour ordering whose tiles'
+// gathered vector fits an SM's shared memory (red_tables; about 8M cells in
+// FP64), on the exact factor.  BiCGStab only in FP64: in FP32 its recurrence
+// turns rounding into a different iteration count in one solve of seven
+// (40 random systems to 1e-5), so FP32 keeps the arithmetic of
+// k_bicg_persistent; so do refinement's inner solves with inner_relax 0 or 1.
+// Solve times, one B200 (per-phase kernels for GMRES, k_bicg_persistent for
+// BiCGStab / reduced form):
+//   GMRES(3) to 1e-3     20k cells 1.29 / 0.27 ms, 1M 4.39 / 0.95, 4M 10.9 / 4.5
+//   BiCGStab to 1e-6     100k cells 1.7 / 0.56 ms, 1M 4.9 / 1.5, 4M 14.0 / 8.4
+// What bounds it: up to 250k cells the exchanges and sums (2 and 3 per
+// BiCGStab iteration, 3 and 4 per GMRES cycle), at 1M the coefficients read
+// from L2 (40 MB per application), at 4M HBM latency at 16 warps per SM.
+template <typename T>
+static bool red_wanted(Solver* S, int nsolv, int maxit) {
+  if (S->opts.multi_kernel || S->opts.ordering != CMS_ORDER_MULTICOLOR || S->cur_relax || S->cur_fuse || maxit < 1 ||
+      maxit > (1 << 26) || (nsolv == 3 && sizeof(T) == 4))
+    return false;
+  return red_tables(S) == CMS_OK && S->rd.state == 1;
+}
+
+// The solve of A x = b (W.b, W.x) by BiCGStab (nsolv 3) or GMRES(3) (nsolv 4)
+// on the factor in A.  Returns 1 when the launch is refused.
+template <typename T>
+static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero) {
+  const HostPattern& P = S->hp;
+  RedTables& R = S->rd;
+  RedBuf& B = red_buf<T>(S);
+  const int n = P.n, g1 = P.gstart[1], nB = n - g1;
+  using P2 = typename Pair<T>::type;
+  if (!B.coef) {
+    P2* c = nullptr;
+    T *cd = nullptr, *gv = nullptr;
+    CHK(S->alloc(&c, (size_t)R.pairs * 32));
+    CHK(S->alloc(&cd, (size_t)nB));
+    CHK(S->alloc(&gv, (size_t)RED_NV_BICG * R.npad));
+    B.coef = c;
+    B.cdiag = cd;
+    B.gvec = gv;
+  }
+  const int nvec = nsolv == 3 ? RED_NV_BICG : RED_NV_GMRES;
+  int nvs = 0, mat = 0;
+  size_t smem = 0;
+  if (!red_plan<T>(R, nvec, R.limit, &nvs, &mat, &smem)) return 1;
+  const double s = sizeof(T);
+  KLAUNCH(S, P_SCHUR_BUILD, (s + 4) * (double)P.nnz_off + 10.0 * n + 8.0 * (double)S->sc_nnz + s * 32.0 * 2 * R.pairs,
+          (k_red_pack<T><<<gsz(nB), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->sc_KC, R.tiles, R.tptr, R.trow, R.slptr,
+                                                         R.sloff, R.mbase, R.ttile, S->d_col, S->d_nlo, S->d_nup,
+                                                         A.aoff, A.diag, S->d_sccol, S->d_sccnt, (P2*)B.coef,
+                                                         (T*)B.cdiag)));
+  RedArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.n = n; a.g1 = g1; a.nB = nB; a.KL = P.KL; a.nt = a.ntiles = R.tiles;
+  a.tptr = R.tptr; a.trow = R.trow; a.tpad = R.tpad; a.rexp = R.rexp; a.kind = R.kind;
+  a.hptr = R.hptr; a.hword = R.hword; a.slptr = R.slptr; a.sloff = R.sloff; a.mbase = R.mbase;
+  a.pcoef = B.coef; a.plcol = R.plcol;
+  a.nphase = R.nphase; a.nfwd = R.nfwd; a.spp = R.spp; a.sprow = R.sprow; a.spe = R.spe; a.spoff = R.spoff;
+  a.spcol = R.spcol; a.osptr = R.osptr; a.osrow = R.osrow;
+  a.luoff = A.luoff; a.invd = A.invd; a.aoff = A.aoff; a.diag = A.diag; a.b = W.b; a.cdiag = (T*)B.cdiag;
+  a.x = W.x; a.rho = W.r;
+  a.col = S->d_col; a.nlo = S->d_nlo; a.nup = S->d_nup;
+  a.gvec = (T*)B.gvec; a.npad = R.npad; a.nvs = nvs; a.mat_smem = mat;
+  a.xw = R.xw; a.slots = R.slots; a.bar = &S->d_st->bar; a.st = S->d_st;
+  a.maxit = maxit; a.norm = norm; a.xzero = xzero; a.tol = tol; a.spin_limit = kSpinLimit;
+  // tags: at most 7 per cycle or iteration; the words are cleared before they run over
+  const unsigned int need = 8u * (unsigned int)maxit + 8u;
+  if (R.tag > 0xffffffffu - need) {
+    CMS_CUDA(cudaMemsetAsync(R.xw, 0, (R.words + 1) * sizeof(ulonglong2), S->stream));
+    CMS_CUDA(cudaMemsetAsync(R.slots, 0, (size_t)2 * (NSMAX * R.tiles + RES_TOT) * sizeof(ulonglong2), S->stream));
+    R.tag = 1;
+  }
+  a.tag0 = R.tag;
+  R.tag += need;
+  CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
+  void* args[] = {&a};
+  prof_begin(S);
+  const void* kern = (const void*)k_red_gmres<T>;
+  if constexpr (sizeof(T) == 8) {
+    if (nsolv == 3) kern = (const void*)k_red_bicg<T>;
+  }
+  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(R.tiles), dim3(RES_BS), args, smem, S->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge) {
+    cudaGetLastError();
+    R.state = -1;
+    return 1;
+  }
+  if (e != cudaSuccess) {
+    std::snprintf(g_last_error, sizeof(g_last_error), "cooperative launch (reduced Krylov): %s", cudaGetErrorString(e));
+    return CMS_DEVICE_ERROR;
+  }
+  S->launches++;
+  const size_t nrec = S->prof_recs.size();
+  prof_end(S, P_PERSIST, 0.0);
+  const bool recorded = S->prof_recs.size() > nrec;
+  CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+  CMS_CUDA(cudaStreamSynchronize(S->stream));
+  if (S->h_st->bar.err) {
+    std::snprintf(g_last_error, sizeof(g_last_error), "reduced Krylov solve: a wait timed out");
+    return CMS_DEVICE_ERROR;
+  }
+  if (recorded) {
+    // C's entries once per operator application; vectors: BiCGStab 26 accesses
+    // of a B row per iteration, GMRES 36 per cycle
+    const double C = (s + 2) * (double)S->sc_nnz;
+    S->prof_recs.back().bytes = nsolv == 3 ? S->h_st->iter * (2 * C + 26.0 * s * nB)
+                                           : S->h_st->inner * C + S->h_st->iter * 36.0 * s * nB;
+  }
+  return CMS_OK;
+}
+
+}  // namespace cms

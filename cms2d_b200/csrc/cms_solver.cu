@@ -22,6 +22,7 @@
 #include "cms_legacy.cuh"
 #include "cms_order.h"
 #include "cms_persist.cuh"
+#include "cms_reduced.cuh"
 #include "cms_resident.cuh"
 #include "cms_schur.cuh"
 #include "cmsgpu.h"
@@ -58,6 +59,24 @@ struct Work {
 template <typename T>
 struct Staging {  // natural-order copies for the host-pointer entry points
   T *acoef = nullptr, *ss = nullptr, *sp = nullptr, *res = nullptr, *phi = nullptr;
+};
+
+// Tables and buffers of the reduced Krylov solves (cms_reduced_host.cuh).
+struct RedTables {
+  int state = 0, tiles = 0, nphase = 0, nfwd = 0, pairs = 0;
+  size_t words = 0, npad = 0, limit = 0;
+  unsigned int tag = 1;  // first tag not used by any launch so far
+  std::vector<int> hb, h_nh, h_nsp, h_ne, h_nos, h_npair;  // per tile: sizes that set the shared memory
+  int *tptr = nullptr, *trow = nullptr, *ttile = nullptr, *tpad = nullptr, *rexp = nullptr, *hptr = nullptr,
+      *hword = nullptr, *slptr = nullptr, *sloff = nullptr, *mbase = nullptr, *spp = nullptr, *spe = nullptr,
+      *spoff = nullptr, *osptr = nullptr, *osrow = nullptr;
+  unsigned short *kind = nullptr, *spcol = nullptr;
+  int2* sprow = nullptr;
+  ushort2* plcol = nullptr;
+  ulonglong2 *xw = nullptr, *slots = nullptr;
+};
+struct RedBuf {  // of one precision
+  void *coef = nullptr, *cdiag = nullptr, *gvec = nullptr;
 };
 
 }  // namespace cms
@@ -117,6 +136,8 @@ struct cms_solver {
   size_t cap_rhrow = 0, cap_rsloff = 0;
   unsigned int rs_tag = 1;  // first tag not used by any launch so far
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
+  cms::RedTables rd;
+  cms::RedBuf rd64, rd32;
   int cur_relax = 0;  // the FP32 factor in A32 is the two-phase one (k_ilu0_relax)
   int cur_fuse = 0;   // inner solves of refinement: update folded into the next iteration
   // MATRIX_SOLVER options 1, 2, 5-8: compass table (built on first use),
@@ -684,6 +705,11 @@ static int run_bicgstab_persistent(Solver* S, Mat<T>& A, Work<T>& W, int tiles, 
   return CMS_OK;
 }
 
+template <typename T>
+static bool red_wanted(Solver* S, int nsolv, int maxit);
+template <typename T>
+static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero);
+
 // BiCGStab from x (or 0) on b, ending when the device stopping test fires.
 template <typename T>
 static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, double tol, int xzero,
@@ -691,6 +717,10 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
   const HostPattern& P = S->hp;
   const int nb_all = S->tab.blk[S->tab.ng];
   if (do_factor) CHK(factor<T>(S, A));
+  if (red_wanted<T>(S, 3, maxit)) {
+    const int rc = run_reduced<T>(S, A, W, 3, maxit, norm, tol, xzero);
+    if (rc != 1) return rc;
+  }
   if (!S->opts.multi_kernel) {
     const int tiles = persist_tiles(S);
     if (tiles > 0) {
@@ -721,11 +751,16 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
 
 // GMRES(3) restarts (pgmres.f90:129-241).
 template <typename T>
-static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bool do_factor = true) {
+static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bool do_factor = true,
+                     bool reduced = true) {
   const HostPattern& P = S->hp;
   const int nb_all = S->tab.blk[S->tab.ng];
   const double vb = (double)P.n * sizeof(T);
   if (do_factor) CHK(factor<T>(S, A));
+  if (reduced && red_wanted<T>(S, 4, maxit)) {
+    const int rc = run_reduced<T>(S, A, W, 4, maxit, 2, tol, 0);
+    if (rc != 1) return rc;
+  }
   KLAUNCH(S, P_SCALAR, 0, (k_gm_start<<<1, 1, 0, S->stream>>>(S->d_st, maxit, tol)));
   GmVecs gv;
   for (int j = 0; j < 5; ++j) gv.v[j] = W.vv[j];
@@ -757,13 +792,14 @@ static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bo
 }
 
 template <typename T>
-static int run_krylov(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero) {
+static int run_krylov(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero,
+                      bool reduced = true) {
   if (nsolv == 3) return run_bicgstab<T>(S, A, W, maxit, norm, tol, xzero);
   if (nsolv == 4) {
     if (xzero) {
       CMS_CUDA(cudaMemsetAsync(W.x, 0, sizeof(T) * S->hp.n, S->stream));
     }
-    return run_gmres<T>(S, A, W, maxit, tol);
+    return run_gmres<T>(S, A, W, maxit, tol, true, reduced);
   }
   return CMS_UNSUPPORTED;
 }
@@ -1235,6 +1271,10 @@ static int resident_count(const Solver* S, int blocks) {
   const int nB = S->hp.n - S->hp.gstart[1];
   return std::max(1, std::min(blocks, (nB + kResRows - 1) / kResRows));
 }
+
+}  // namespace cms
+#include "cms_reduced_host.cuh"
+namespace cms {
 
 // The automatic layout of the reduced inner solve on a multicolour ordering:
 // the resident form where the system fits it.
