@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "cms_common.cuh"
+#include "cms_gmres_cluster.cuh"
 #include "cms_krylov.cuh"
 #include "cms_legacy.cuh"
 #include "cms_order.h"
@@ -74,6 +75,11 @@ struct RedTables {
   int2* sprow = nullptr;
   ushort2* plcol = nullptr;
   ulonglong2 *xw = nullptr, *slots = nullptr;
+};
+struct GmcPlan {  // launch of GMRES as one cluster: 0 not planned, 1 planned, -1 not possible
+  int state = 0, nc = 0, stage = 0;
+  size_t smem = 0;
+  const void* kern = nullptr;
 };
 struct RedBuf {  // of one precision
   void *coef = nullptr, *cdiag = nullptr, *gvec = nullptr;
@@ -138,6 +144,7 @@ struct cms_solver {
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   cms::RedTables rd;
   cms::RedBuf rd64, rd32;
+  cms::GmcPlan gmc[2];  // FP32, FP64
   int cur_relax = 0;  // the FP32 factor in A32 is the two-phase one (k_ilu0_relax)
   int cur_fuse = 0;   // inner solves of refinement: update folded into the next iteration
   // MATRIX_SOLVER options 1, 2, 5-8: compass table (built on first use),
@@ -749,6 +756,76 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
   return CMS_OK;
 }
 
+// GMRES(3) of a small system as one cluster launch (cms_gmres_cluster.cuh),
+// with the rounding of the per-phase kernels.  Returns 1 when the system or
+// the device does not take it.
+template <typename T>
+static int run_gmres_cluster(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol) {
+  const HostPattern& P = S->hp;
+  GmcPlan& L = S->gmc[sizeof(T) == 8 ? 1 : 0];
+  if (L.state < 0) return 1;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(GMC_BS);
+  cfg.stream = S->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (L.state == 0) {  // the launch's shape, once per handle and precision
+    L.state = -1;
+    if (P.n > GMC_ROWS || P.G > 8 || P.G < 1 || S->tab.ng != P.G || S->tab.blk[S->tab.ng] > GMC_PART ||
+        P.gkl[0] != 0)
+      return 1;
+    int nslot = 0;
+    for (int r = 0; r < P.n; ++r) nslot = std::max(nslot, P.nlo[r] + P.nup[r]);
+    if (nslot > 8) return 1;
+    L.kern = gmc_kernel<T>(nslot);
+    int optin = 0;
+    cudaFuncAttributes fa;
+    CMS_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S->dev));
+    CMS_CUDA(cudaFuncGetAttributes(&fa, L.kern));
+    L.nc = 1;
+    while (L.nc < 16 && L.nc * GMC_BS < P.n) L.nc *= 2;
+    const size_t rows = (size_t)((S->tab.blk[S->tab.ng] + L.nc - 1) / L.nc) * TPB, ns = nslot <= 4 ? 4 : nslot <= 6 ? 6 : 8;
+    const size_t limit = (size_t)optin - fa.sharedSizeBytes;
+    const size_t s0 = rows * (2 * sizeof(T) + 1), s1 = s0 + rows * ns * (sizeof(T) + sizeof(int)),
+                 s2 = s1 + rows * ns * sizeof(T);
+    if (s0 > limit) return 1;
+    L.stage = s2 <= limit ? 2 : s1 <= limit ? 1 : 0;
+    L.smem = L.stage == 2 ? s2 : L.stage == 1 ? s1 : s0;
+    CMS_CUDA(cudaFuncSetAttribute(L.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    CMS_CUDA(cudaFuncSetAttribute(L.kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    at[0].val.clusterDim.x = L.nc;
+    cfg.gridDim = dim3(L.nc);
+    cfg.dynamicSmemBytes = L.smem;
+    int fit = 0;
+    if (cudaOccupancyMaxActiveClusters(&fit, L.kern, &cfg) != cudaSuccess || fit < 1) {
+      cudaGetLastError();
+      return 1;
+    }
+    L.state = 1;
+  }
+  GmcArgs<T> a;
+  std::memset(&a, 0, sizeof(a));
+  a.n = P.n; a.KL = P.KL; a.maxit = maxit; a.stage = L.stage; a.tol = tol; a.tab = S->tab;
+  a.gku_last = P.gku[P.G - 1];
+  a.col = S->d_col; a.nlo = S->d_nlo; a.nup = S->d_nup;
+  a.aoff = A.aoff; a.diag = A.diag; a.luoff = A.luoff; a.invd = A.invd; a.b = W.b; a.x = W.x; a.z = W.z;
+  for (int j = 0; j < 4; ++j) a.vh[j] = W.vv[j + 1];
+  a.vs[0] = W.p; a.vs[1] = W.u; a.vs[2] = W.v;
+  a.st = S->d_st;
+  at[0].val.clusterDim.x = L.nc;
+  cfg.gridDim = dim3(L.nc);
+  cfg.dynamicSmemBytes = L.smem;
+  prof_begin(S);
+  void* args[] = {&a};
+  CMS_CUDA(cudaLaunchKernelExC(&cfg, L.kern, args));
+  S->launches++;
+  prof_end(S, P_PERSIST, 0.0);
+  return CMS_OK;
+}
+
 // GMRES(3) restarts (pgmres.f90:129-241).
 template <typename T>
 static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bool do_factor = true,
@@ -759,6 +836,10 @@ static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bo
   if (do_factor) CHK(factor<T>(S, A));
   if (reduced && red_wanted<T>(S, 4, maxit)) {
     const int rc = run_reduced<T>(S, A, W, 4, maxit, 2, tol, 0);
+    if (rc != 1) return rc;
+  }
+  if (!S->opts.multi_kernel) {
+    const int rc = run_gmres_cluster<T>(S, A, W, maxit, tol);
     if (rc != 1) return rc;
   }
   KLAUNCH(S, P_SCALAR, 0, (k_gm_start<<<1, 1, 0, S->stream>>>(S->d_st, maxit, tol)));
