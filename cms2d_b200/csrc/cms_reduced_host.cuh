@@ -36,12 +36,25 @@ static bool red_plan(const RedTables& R, int nvec, size_t limit, int* nvs, int* 
   return true;
 }
 
+// Vectors of the streamed reduced solve (cms_schur_stream.cuh) that fit in
+// shared memory beside the gathered ones, -1 when those do not; the launch's
+// shared memory.
+static int stream_vectors(const RedTables& R, size_t limit, size_t* smem) {
+  for (int v = SV_N; v >= 0; --v) {
+    size_t most = 0;
+    for (int t = 0; t < R.tiles; ++t) most = std::max(most, stream_smem(R.hb[t], R.h_nh[t], v));
+    *smem = most;
+    if (most <= limit) return v;
+  }
+  return -1;
+}
+
 // Dynamic shared memory the kernels may use, set as their attribute.
 static int red_limit(Solver* S, size_t* limit) {
   int optin = 0;
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S->dev) != cudaSuccess) return CMS_DEVICE_ERROR;
-  const void* k[3] = {(const void*)k_red_bicg<double>, (const void*)k_red_gmres<double>,
-                      (const void*)k_red_gmres<float>};
+  const void* k[4] = {(const void*)k_red_bicg<double>, (const void*)k_red_gmres<double>,
+                      (const void*)k_red_gmres<float>, (const void*)k_schur_stream};
   size_t most = (size_t)optin;
   for (const void* f : k) {
     cudaFuncAttributes fa;
@@ -120,6 +133,7 @@ static int red_tables(Solver* S) {
   R.h_nos.assign(nt, 0);
   R.h_npair.assign(nt, 0);
   std::vector<ushort2> plcol;
+  std::vector<int2> ppos(nB);
   std::vector<int> touched, stack;
   int pairs = 0, pad = 0;
   for (int t = 0; t < nt; ++t) {
@@ -206,6 +220,7 @@ static int red_tables(Solver* S) {
       plcol.resize(base + (size_t)w * 32);
       for (int l = 0; l < 32; ++l) {
         const int k = j * 32 + l, i = k < nb[t] ? trow[tptr[t] + k] : -1;
+        if (i >= 0) ppos[i] = make_int2((int)base + l, w);
         const unsigned short own = (unsigned short)std::min(k, nb[t] - 1);
         for (int q = 0; q < w; ++q) {
           auto lc = [&](int s) {
@@ -226,7 +241,7 @@ static int red_tables(Solver* S) {
   size_t limit = 0, smem = 0;
   CHK(red_limit(S, &limit));
   int nvs, mat;
-  if (!red_plan<double>(R, RED_NV_BICG, limit, &nvs, &mat, &smem)) return CMS_OK;
+  if (!red_plan<double>(R, RED_NV_BICG, limit, &nvs, &mat, &smem) && stream_vectors(R, limit, &smem) < 0) return CMS_OK;
   // words: a tile's are consecutive, on lines of their own
   size_t words = 0;
   std::vector<int> rexp(nB, -1);
@@ -255,6 +270,7 @@ static int red_tables(Solver* S) {
   CHK(put(&R.sloff, sloff));
   CHK(put(&R.mbase, mbase));
   CHK(put(&R.plcol, plcol));
+  CHK(put(&R.ppos, ppos));
   CHK(put(&R.spp, spp));
   CHK(put(&R.sprow, sprow));
   CHK(put(&R.spe, spe));
@@ -275,9 +291,59 @@ static int red_tables(Solver* S) {
   return CMS_OK;
 }
 
+// need tags for a launch; the words are cleared before the 32-bit tags run over.
+static int red_tags(Solver* S, unsigned int need, unsigned int* tag0) {
+  RedTables& R = S->rd;
+  if (R.tag > 0xffffffffu - need) {
+    CMS_CUDA(cudaMemsetAsync(R.xw, 0, (R.words + 1) * sizeof(ulonglong2), S->stream));
+    CMS_CUDA(cudaMemsetAsync(R.slots, 0, (size_t)2 * (NSMAX * R.tiles + RES_TOT) * sizeof(ulonglong2), S->stream));
+    if (S->st_xnu) CMS_CUDA(cudaMemsetAsync(S->st_xnu, 0, (R.words + 1) * sizeof(unsigned long long), S->stream));
+    R.tag = 1;
+  }
+  *tag0 = R.tag;
+  R.tag += need;
+  return CMS_OK;
+}
+
 template <typename T>
 static RedBuf& red_buf(Solver* S) {
   return sizeof(T) == 8 ? S->rd64 : S->rd32;
+}
+
+// Whether the reduced inner solve of refinement streams (the automatic layout,
+// too large for the resident form, the gathered vectors fit; up to about 8M
+// cells); allocates its buffers.  Kernel time per iteration, one B200,
+// telescoping systems, form of cms_schur.cuh / streamed: 1.3M cells 42.7 / 19.9
+// us, 2.0M 87.3 / 27.4, 4.0M 156 / 66, 7.3M 280 / 150.  Bound by HBM at 4M and
+// above (about 70 % of the measured copy rate).
+static bool stream_choose(Solver* S) {
+  if (red_tables(S) != CMS_OK || S->rd.state != 1) return false;
+  RedTables& R = S->rd;
+  size_t smem = 0;
+  if (stream_vectors(R, R.limit, &smem) < 0) return false;
+  if (!S->st_coef &&
+      (S->alloc(&S->st_coef, (size_t)R.pairs * 32) || S->alloc(&S->st_vec, (size_t)SV_N * R.npad) ||
+       S->alloc(&S->st_xnu, R.words + 1)))
+    return false;
+  return true;
+}
+
+// Its arguments beyond the system's (tags from the tables' words).
+static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
+  RedTables& R = S->rd;
+  a->tptr = R.tptr; a->trow = R.trow; a->tpad = R.tpad; a->rexp = R.rexp; a->hptr = R.hptr; a->hword = R.hword;
+  a->slptr = R.slptr; a->sloff = R.sloff; a->mbase = R.mbase;
+  a->pcoef = S->st_coef; a->plcol = R.plcol; a->gvec = S->st_vec; a->npad = R.npad;
+  a->nvs = stream_vectors(R, R.limit, smem);
+  // what L2 keeps of the matrix beside the vectors of global memory: of 126 MB,
+  // 75 (per iteration at 2.9M cells: 48.7 us with every slice evict-first, 44.7
+  // with 60-80 MB kept, 54.2 with 100 MB; at 2.0M 35.7, 27.4, 27.4; at 4.0M
+  // 66.4, 66.1-67.3, 75.0)
+  const double mat = 32.0 * R.pairs * (sizeof(float2) + sizeof(ushort2)), vecs = (SV_N - a->nvs) * 4.0 * (double)R.npad;
+  constexpr double kL2Keep = 75e6;
+  a->keep = (float)std::min(1.0, std::max(0.0, (kL2Keep - vecs) / mat));
+  a->xst = R.xw; a->xnu = S->st_xnu; a->slots = R.slots;
+  return red_tags(S, (unsigned int)maxit + 2u, &a->S.tag0);
 }
 
 // Whether a solve runs in reduced form: a multicolour ordering whose tiles'
@@ -344,15 +410,7 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   a.gvec = (T*)B.gvec; a.npad = R.npad; a.nvs = nvs; a.mat_smem = mat;
   a.xw = R.xw; a.slots = R.slots; a.bar = &S->d_st->bar; a.st = S->d_st;
   a.maxit = maxit; a.norm = norm; a.xzero = xzero; a.tol = tol; a.spin_limit = kSpinLimit;
-  // tags: at most 7 per cycle or iteration; the words are cleared before they run over
-  const unsigned int need = 8u * (unsigned int)maxit + 8u;
-  if (R.tag > 0xffffffffu - need) {
-    CMS_CUDA(cudaMemsetAsync(R.xw, 0, (R.words + 1) * sizeof(ulonglong2), S->stream));
-    CMS_CUDA(cudaMemsetAsync(R.slots, 0, (size_t)2 * (NSMAX * R.tiles + RES_TOT) * sizeof(ulonglong2), S->stream));
-    R.tag = 1;
-  }
-  a.tag0 = R.tag;
-  R.tag += need;
+  CHK(red_tags(S, 8u * (unsigned int)maxit + 8u, &a.tag0));  // at most 7 per cycle or iteration
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   void* args[] = {&a};
   prof_begin(S);

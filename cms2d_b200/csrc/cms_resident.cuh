@@ -219,6 +219,32 @@ struct ResState {
   int it_best, converged, nonfinite;
 };
 
+// The start, from r0.r0 and f0.r0.
+__device__ __forceinline__ void resident_first(double rr, double fr, double tol, ResState& st, ResScal& sc) {
+  const double res0 = sqrt(rr);
+  st.res0 = res0;
+  st.rho = st.rr_last = st.best2 = rr;
+  st.tol2 = (tol * res0) * (tol * res0);
+  st.it_best = 0;
+  st.converged = res0 == 0.0 ? 1 : 0;
+  st.nonfinite = res0 != 0.0 && (!isfinite(fr) || !isfinite(res0)) ? 1 : 0;
+  st.alf = res0 != 0.0 && !st.nonfinite && fr != 0.0 ? rr / fr : 0.0;
+  sc.ay = (float)st.alf;
+  // a breakdown before the first step (f0.r0 = 0) stops with x = 0
+  sc.stop = (st.converged || st.nonfinite || fr == 0.0 ? 1 : 0) | (st.nonfinite ? 2 : 0);
+}
+
+// The solve's record: last: the result is the last iterate, not the best one.
+__device__ __forceinline__ void resident_report(DevState* d, const ResState& st, int it, int nonfinite, bool last) {
+  const double rr = !nonfinite && !last ? st.best2 : st.rr_last;
+  d->iter = it;
+  d->s[S_RELRES] = nonfinite ? rr : st.res0 > 0.0 ? sqrt(rr) / st.res0 : 0.0;
+  d->s[S_RES0] = st.res0;
+  d->converged = st.converged;
+  d->nonfinite = nonfinite;
+  d->done = 1;
+}
+
 // omg of an iteration, by every thread.
 __device__ __forceinline__ double resident_omega(const double* t) {
   const double d = fmax(t[1], SMALL);
@@ -452,17 +478,7 @@ __device__ __forceinline__ void schur_body_resident(const SchurArgs& A) {
   publish_sums<2, RES_NW>(s2, act, s_sum, A.slots, nt, tile, 0, base);
   ph.ok = !__syncthreads_or(!ph.ok | collect_sums<2, RES_NW>(s_bc, A.slots, tot, nt, tile, 0, base, A.bar, A.spin_limit));
   if (threadIdx.x == 0) {
-    const double rr = s_bc[0], fr = s_bc[1], res0 = sqrt(rr);
-    s_st.res0 = res0;
-    s_st.rho = s_st.rr_last = s_st.best2 = rr;
-    s_st.tol2 = (A.tol * res0) * (A.tol * res0);
-    s_st.it_best = 0;
-    s_st.converged = res0 == 0.0 ? 1 : 0;
-    s_st.nonfinite = res0 != 0.0 && (!isfinite(fr) || !isfinite(res0)) ? 1 : 0;
-    s_st.alf = res0 != 0.0 && !s_st.nonfinite && fr != 0.0 ? rr / fr : 0.0;
-    s_sc.ay = (float)s_st.alf;
-    // a breakdown before the first step (f0.r0 = 0) stops with x = 0
-    s_sc.stop = (s_st.converged || s_st.nonfinite || fr == 0.0 ? 1 : 0) | (s_st.nonfinite ? 2 : 0);
+    resident_first(s_bc[0], s_bc[1], A.tol, s_st, s_sc);
   }
   __syncthreads();
   int it = 0, nonfinite = (s_sc.stop & 2) ? 1 : 0;
@@ -569,15 +585,7 @@ __device__ __forceinline__ void schur_body_resident(const SchurArgs& A) {
       }
     }
   }
-  if (tile == 0 && threadIdx.x == 0) {
-    A.st->iter = it;
-    const double rr = !nonfinite && !last ? s_st.best2 : s_st.rr_last;
-    A.st->s[S_RELRES] = nonfinite ? rr : s_st.res0 > 0.0 ? sqrt(rr) / s_st.res0 : 0.0;
-    A.st->s[S_RES0] = s_st.res0;
-    A.st->converged = s_st.converged;
-    A.st->nonfinite = nonfinite;
-    A.st->done = 1;
-  }
+  if (tile == 0 && threadIdx.x == 0) resident_report(A.st, s_st, it, nonfinite, last);
 }
 
 // One system: block b works on tile b.

@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(TPB, 4) k_schur_off(int n, int g1, int nB, int
                                                    const signed char* __restrict__ nup,
                                                    const float* __restrict__ aoff, const float* __restrict__ diag,
                                                    const float* __restrict__ sinv, const int* __restrict__ ccol,
-                                                   const signed char* __restrict__ ccnt, float* __restrict__ coff) {
+                                                   const signed char* __restrict__ ccnt, float* __restrict__ coff,
+                                                   const int2* __restrict__ ppos, float2* __restrict__ pcoef) {
   __shared__ double s_acc[KSC][TPB];  // this thread's columns and accumulators: column threadIdx.x
   __shared__ int s_cc[KSC][TPB];
   double* acc = &s_acc[0][threadIdx.x];
@@ -182,6 +183,13 @@ __global__ void __launch_bounds__(TPB, 4) k_schur_off(int n, int g1, int nB, int
     }
     for (int q = 0; q < KC; ++q)
       coff[(size_t)q * nB + i] = q < kc ? (float)(acc[q * TPB] * (double)sinv[cc[q * TPB]]) : 0.0f;
+    if (pcoef) {  // the packed slices too (cms_schur_stream.cuh): first pair and number of pairs
+      const int2 pp = ppos[i];
+      for (int q = 0; q < pp.y; ++q)
+        pcoef[(size_t)pp.x + (size_t)q * 32] =
+            make_float2(2 * q < KC ? coff[(size_t)(2 * q) * nB + i] : 0.0f,
+                        2 * q + 1 < KC ? coff[(size_t)(2 * q + 1) * nB + i] : 0.0f);
+    }
   }
 }
 

@@ -26,6 +26,7 @@
 #include "cms_reduced.cuh"
 #include "cms_resident.cuh"
 #include "cms_schur.cuh"
+#include "cms_schur_stream.cuh"
 #include "cmsgpu.h"
 
 static char g_last_error[512] = "";
@@ -74,6 +75,7 @@ struct RedTables {
   unsigned short *kind = nullptr, *spcol = nullptr;
   int2* sprow = nullptr;
   ushort2* plcol = nullptr;
+  int2* ppos = nullptr;  // [nB] a row's first packed pair, pairs of its slice
   ulonglong2 *xw = nullptr, *slots = nullptr;
 };
 struct GmcPlan {  // launch of GMRES as one cluster: 0 not planned, 1 planned, -1 not possible
@@ -144,6 +146,9 @@ struct cms_solver {
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   cms::RedTables rd;
   cms::RedBuf rd64, rd32;
+  float2* st_coef = nullptr;  // streamed reduced solve: packed Chat, vectors, words of nu
+  float* st_vec = nullptr;
+  unsigned long long* st_xnu = nullptr;
   cms::GmcPlan gmc[2];  // FP32, FP64
   int cur_relax = 0;  // the FP32 factor in A32 is the two-phase one (k_ilu0_relax)
   int cur_fuse = 0;   // inner solves of refinement: update folded into the next iteration
@@ -1266,7 +1271,7 @@ static int resident_tables(Solver* S, int tiles) {
 }
 
 // Chat's values and sinv from the FP32 matrix (once per solve).
-static int schur_numeric(Solver* S) {
+static int schur_numeric(Solver* S, bool packed = false) {
   const HostPattern& P = S->hp;
   const int n = P.n, g1 = P.gstart[1], nB = n - g1;
   const double nnz = (double)P.nnz_off;
@@ -1276,7 +1281,8 @@ static int schur_numeric(Solver* S) {
   KLAUNCH(S, P_SCHUR_BUILD, 8.0 * nnz + 10.0 * n + 4.0 * n + 8.0 * (double)S->sc_nnz + nB,
           (k_schur_off<<<gsz(nB), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->sc_KC, S->d_col, S->d_nlo, S->d_nup,
                                                         S->A32.aoff, S->A32.diag, S->d_ssinv, S->d_sccol,
-                                                        S->d_sccnt, S->d_scoff)));
+                                                        S->d_sccnt, S->d_scoff, packed ? S->rd.ppos : nullptr,
+                                                        packed ? S->st_coef : nullptr)));
   return CMS_OK;
 }
 
@@ -1406,19 +1412,29 @@ static int schur_tiles(Solver* S, int layout) {
 }
 
 // The reduced FP32 inner solve (W32.b -> W32.x) as one cooperative launch.
-static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, bool resident) {
+enum SchurForm : int { SF_TILES = 0, SF_RESIDENT = 1, SF_STREAM = 2 };
+static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, SchurForm form) {
+  const bool resident = form == SF_RESIDENT;
   if (resident) tiles = S->rs_tiles;
+  if (form == SF_STREAM) tiles = S->rd.tiles;
   SchurArgs a = make_schur_args(S, tiles, maxit, tol);
   const SchurLayout L = schur_layout(schur_layout_run(S));
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
+  StreamArgs sa;
+  size_t ssmem = 0;
   if (resident)
     CHK(resident_tags(S, maxit, &a.tag0));
-  else
+  else if (form == SF_STREAM) {
+    sa.S = a;
+    CHK(stream_args(S, maxit, &sa, &ssmem));
+  } else
     CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
-  void* args[] = {&a};
+  void* args[] = {form == SF_STREAM ? (void*)&sa : (void*)&a};
   prof_begin(S);
   const cudaError_t e =
-      resident ? cudaLaunchCooperativeKernel(resident_kernel(S->rs_nr, false), dim3(tiles), dim3(RES_BS), args,
+      form == SF_STREAM ? cudaLaunchCooperativeKernel((const void*)k_schur_stream, dim3(tiles), dim3(STR_BS), args,
+                                                      ssmem, S->stream)
+      : resident ? cudaLaunchCooperativeKernel(resident_kernel(S->rs_nr, false), dim3(tiles), dim3(RES_BS), args,
                                              S->rs_smem, S->stream)
                : cudaLaunchCooperativeKernel(L.single, dim3(tiles), dim3(L.bs), args, 0, S->stream);
   if (e != cudaSuccess) {
@@ -1560,8 +1576,12 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
   const bool mc_persist = nsolv == 3 && S->opts.ordering == CMS_ORDER_MULTICOLOR && !S->opts.multi_kernel &&
                           persist_tiles(S) > 0;
   bool schur = mc_persist && S->opts.inner_relax == 2;
-  const bool resident = schur && resident_choose(S);
-  if (schur && !resident) {  // the tiles of the reduced kernel's layout
+  // resident on the SMs, else streamed, else the tiles of the layout option
+  const SchurForm form = !schur ? SF_TILES
+                         : resident_choose(S) ? SF_RESIDENT
+                         : resident_wanted(S) && schur_pattern(S) == CMS_OK && S->sc_sym && stream_choose(S) ? SF_STREAM
+                                                                                                            : SF_TILES;
+  if (schur && form == SF_TILES) {  // the tiles of the reduced kernel's layout
     const int nt = schur_tiles(S, schur_layout_index(S));
     schur = nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->ptiles) == CMS_OK;
   }
@@ -1572,7 +1592,7 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
   } relax_scope{S};
   S->cur_fuse = 1;
   if (schur) {
-    CHK(schur_numeric(S));
+    CHK(schur_numeric(S, form == SF_STREAM));
   } else if (relax) {
     KLAUNCH(S, P_ILU0, (double)n * (3 * 4 + 2) + (double)(P.nnz_off) * (2 * 4 + 4),
             (k_ilu0_relax<float><<<gsz(n), TPB, 0, S->stream>>>(n, P.KL, P.gstart[1], S->d_col, S->d_nlo,
@@ -1599,7 +1619,7 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
     refine_inner_limits(S->opts, R);
     KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
     if (schur) {
-      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, resident));  // tiles built above for its layout
+      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, form));  // tiles built above for its layout
     } else if (nsolv == 3) {
       CHK(run_bicgstab<float>(S, S->A32, S->W32, R.imax, 2, R.itol, 1, false));
     } else {

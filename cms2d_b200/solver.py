@@ -76,8 +76,9 @@ class Solver:
                the solve's remaining iteration budget and is asked for
                0.5 tol / (outer residual so far) within [1e-6, 1e-3].
     reduced_layout: block/row layout and iteration form of the reduced inner
-               solve (0 auto: resident on the SMs up to about 1M cells, else 1024
-               threads x 2 rows, single reduction; cms_solver_opts.reduced_layout).
+               solve (0 auto: resident on the SMs up to about 1M cells, streamed up to
+               about 8M, else 1024 threads x 2 rows, single reduction;
+               cms_solver_opts.reduced_layout).
     """
 
     def __init__(self, grid, iwet=None, ordering: str = "multicolor", precision: str = "fp64", tol: float = 1e-3,

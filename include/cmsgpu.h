@@ -87,7 +87,8 @@ typedef struct cms_solver_opts {
   int reduced_layout; /* block and row layout of the reduced inner solve: 0 auto
                         (the resident form, one block per SM with its tile's system
                         in shared memory and registers, where every tile fits: up to
-                        about 1M cells on one B200; else 5), 1 256 threads x 2 rows, 2 512 x 2, 3 512 x 4, 4 1024 x 2
+                        about 1M cells on one B200; its streamed form up to about 8M;
+                        else 5), 1 256 threads x 2 rows, 2 512 x 2, 3 512 x 4, 4 1024 x 2
                         (three phases, two grid barriers per iteration); 5 1024 x 2,
                         6 512 x 2, 7 256 x 2 in the single-reduction form (one
                         barrier per iteration; needs a structurally symmetric

@@ -3,7 +3,8 @@
 Sizes: a single partial slice of 32 rows, one tile, tiles cut just below and
 above a multiple of the rows per tile, a strip narrower than a tile, islands
 (a grid in several pieces), telescoping interfaces, two and four rows per
-thread, and a system just too large for the SMs (the streaming form).  Each
+thread, and systems too large for the SMs (the streamed form, with all, some and none
+of its vectors in shared memory).  Each
 solution is compared with a direct FP64 solve; the stopping test asks for a
 1e-10 residual, |A^-1| is at most 1 / (0.02 * 0.2) = 250 (diagonal 1.02 times
 a row sum of at least two coefficients of 0.1) and |b| / |x|_max at most
@@ -67,10 +68,11 @@ def test_resident_matches_direct_solve(kind):
     assert np.abs(x - ref).max() <= 1e-10 * 250 * np.sqrt(n) * np.abs(ref).max(), info
 
 
-@pytest.mark.parametrize("kind, cells", [("cart", 330_000), ("tel", 500_000), ("cart", 1_160_000), ("cart", 1_300_000)])
+@pytest.mark.parametrize("kind, cells", [("cart", 330_000), ("tel", 500_000), ("cart", 1_160_000), ("cart", 1_300_000),
+                                         ("tel", 2_000_000), ("cart", 5_600_000)])
 def test_resident_rows_per_thread(kind, cells):
-    """Two, four and eight rows per thread, and the streaming form beyond: the
-    FP64 residual of the result, and the streaming form's solution."""
+    """Two, four and eight rows per thread, and the streamed form beyond: the
+    FP64 residual of the result, and the solution of the 1024 x 2 layout."""
     side = int(round(cells ** 0.5))
     g = G.cartesian_grid(side, side) if kind == "cart" else G.solver_test_grid(cells)
     *_, (info, x) = _solve(g, 22)
