@@ -92,71 +92,104 @@ template <typename T> struct Pair;
 template <> struct Pair<double> { using type = double2; };
 template <> struct Pair<float> { using type = float2; };
 
-// C's coefficients in the packed order (one thread per B row, tile order), its
-// diagonal, from A:  C_ik = a_ik - sum_j a_ij a_jk / d_j (A's off-diagonals
-// are -aoff; coff = -C_ik), sums in FP64.
-template <typename T>
-__global__ void __launch_bounds__(TPB, 4) k_red_pack(int n, int g1, int nB, int KL, int KC, int nt,
-                                                     const int* __restrict__ tptr, const int* __restrict__ trow,
-                                                     const int* __restrict__ slptr, const int* __restrict__ sloff,
-                                                     const int* __restrict__ mbase, const int* __restrict__ ttile,
-                                                     const int* __restrict__ col, const signed char* __restrict__ nlo,
+// C's coefficients in the packed slices and its diagonal, from A
+// (coff = -C_ik, sums in FP64), and the part of the ILU(0) factor that the
+// solve needs: 1/C_rr for the rows without couplings among B rows, whose
+// factor row that is; for the special rows C's values at A's couplings among B
+// rows, which are the final upper entries of a group-1 row and the start of the
+// others' elimination (k_red_special).  (This and k_red_special replace a
+// factorisation of all rows, one launch per group: at 1M cells FP64 117 us and
+// 71 us for the coefficients; now 55 us together.)
+template <typename T, int KS>
+__global__ void __launch_bounds__(TPB, 4) k_red_pack(int n, int g1, int nB, int KL, const int* __restrict__ col,
+                                                     const signed char* __restrict__ nlo,
                                                      const signed char* __restrict__ nup, const T* __restrict__ aoff,
-                                                     const T* __restrict__ diag, const int* __restrict__ ccol,
+                                                     const T* __restrict__ diag, SchurMap M,
                                                      const signed char* __restrict__ ccnt,
+                                                     const int2* __restrict__ ppos,
                                                      typename Pair<T>::type* __restrict__ pcoef,
-                                                     T* __restrict__ cdiag) {
+                                                     T* __restrict__ cdiag, T* __restrict__ luoff,
+                                                     T* __restrict__ invd) {
   __shared__ double s_acc[KSC][TPB];
-  __shared__ int s_cc[KSC][TPB];
   double* acc = &s_acc[0][threadIdx.x];
-  int* cc = &s_cc[0][threadIdx.x];
-  for (int p = blockIdx.x * TPB + threadIdx.x; p < nB; p += gridDim.x * TPB) {
-    const int t = __ldg(ttile + p), k = p - __ldg(tptr + t), i = __ldg(trow + p), r = g1 + i;
-    const int kc = ccnt[i];
-    for (int q = 0; q < kc; ++q) {
-      cc[q * TPB] = ccol[(size_t)q * nB + i];
-      acc[q * TPB] = 0.0;
-    }
+  for (int i = blockIdx.x * TPB + threadIdx.x; i < nB; i += gridDim.x * TPB) {
+    const int r = g1 + i, kc = ccnt[i], kl = nlo[r], kt = kl + nup[r];
+    for (int q = 0; q < kc; ++q) acc[q * TPB] = 0.0;
     double d = diag[r];
-    const int kl = nlo[r], ku = nup[r];
-    for (int s = 0; s < kl + ku; ++s) {
-      const size_t e = (size_t)(s < kl ? s : KL + (s - kl)) * n + r;
-      const int j = col[e];
-      const double a = aoff[e];
-      if (j >= g1) {
-        for (int q = 0; q < kc; ++q)
-          if (cc[q * TPB] == j) {
-            acc[q * TPB] += a;
-            break;
-          }
-        continue;
-      }
-      const double w = a / (double)diag[j];
-      const int nuj = nup[j];
-      for (int t2 = 0; t2 < nuj; ++t2) {
-        const size_t e2 = (size_t)(KL + t2) * n + j;
-        const int k2 = col[e2];
-        const double v = w * (double)aoff[e2];
-        if (k2 == r) {
-          d -= v;
-          continue;
-        }
-        for (int q = 0; q < kc; ++q)
-          if (cc[q * TPB] == k2) {
-            acc[q * TPB] += v;
-            break;
-          }
-      }
-    }
+    schur_row<T, KS>(n, g1, nB, KL, i, kl, kt, col, aoff, diag, M.smap, acc, d);
     cdiag[i] = (T)d;
-    const int* so = sloff + __ldg(slptr + t) + (k >> 5);
-    const int o = __ldg(so), wid = __ldg(so + 1) - o;
-    typename Pair<T>::type* out = pcoef + ((size_t)__ldg(mbase + t) + o) * 32 + (k & 31);
-    for (int q = 0; q < wid; ++q) {
+    invd[r] = (T)(1.0 / d);
+    for (int c = 0; c < kt; ++c) {
+      const size_t e = (size_t)(c < kl ? c : KL + (c - kl)) * n + r;
+      if (__ldg(col + e) >= g1) luoff[e] = (T)-acc[(int)(__ldg(M.smap + (size_t)c * nB + i) & 0xff) * TPB];
+    }
+    const int2 pp = ppos[i];
+    for (int q = 0; q < pp.y; ++q) {
       typename Pair<T>::type v;
       v.x = 2 * q < kc ? (T)acc[2 * q * TPB] : T(0);
       v.y = 2 * q + 1 < kc ? (T)acc[(2 * q + 1) * TPB] : T(0);
-      out[(size_t)q * 32] = v;
+      pcoef[(size_t)pp.x + (size_t)q * 32] = v;
+    }
+  }
+}
+
+// ILU(0) elimination among B rows for the special rows of group g >= 2 (rows
+// in list): k_ilu0's steps on the couplings to B rows, the couplings to group
+// 0 already eliminated.
+template <typename T>
+__global__ void __launch_bounds__(TPB) k_red_special(int n, int g1, int KL, int count, const int* __restrict__ list,
+                                                     const int* __restrict__ col, const signed char* __restrict__ nlo,
+                                                     const signed char* __restrict__ nup, const T* __restrict__ cdiag,
+                                                     T* luoff, T* invd) {
+  for (int p = blockIdx.x * TPB + threadIdx.x; p < count; p += gridDim.x * TPB) {
+    const int r = list[p], kl = nlo[r], ku = nup[r];
+    T al[KMAX], au[KMAX];
+    int cl[KMAX], cu[KMAX];
+#pragma unroll
+    for (int s = 0; s < KMAX; ++s) {
+      cl[s] = cu[s] = -1;
+      al[s] = au[s] = T(0);
+      if (s < kl) {
+        const int c = col[(size_t)s * n + r];
+        if (c >= g1) {
+          cl[s] = c;
+          al[s] = luoff[(size_t)s * n + r];
+        }
+      }
+      if (s < ku) {
+        cu[s] = col[(size_t)(KL + s) * n + r];
+        au[s] = luoff[(size_t)(KL + s) * n + r];
+      }
+    }
+    T d = cdiag[r - g1];
+#pragma unroll
+    for (int s = 0; s < KMAX; ++s) {
+      const int j = cl[s];
+      if (j < 0) continue;
+      const T lij = al[s] * invd[j];
+      al[s] = lij;
+      const int nuj = nup[j];
+#pragma unroll 1
+      for (int t2 = 0; t2 < nuj; ++t2) {
+        const int k = col[(size_t)(KL + t2) * n + j];
+        const T ujk = luoff[(size_t)(KL + t2) * n + j];
+        if (k == r) {
+          d = d - lij * ujk;
+        } else {
+#pragma unroll
+          for (int s2 = s + 1; s2 < KMAX; ++s2)
+            if (cl[s2] == k) al[s2] = al[s2] - lij * ujk;
+#pragma unroll
+          for (int t = 0; t < KMAX; ++t)
+            if (cu[t] == k) au[t] = au[t] - lij * ujk;
+        }
+      }
+    }
+    invd[r] = T(1) / d;
+#pragma unroll
+    for (int s = 0; s < KMAX; ++s) {
+      if (s < kl && cl[s] >= 0) luoff[(size_t)s * n + r] = al[s];
+      if (s < ku) luoff[(size_t)(KL + s) * n + r] = au[s];
     }
   }
 }

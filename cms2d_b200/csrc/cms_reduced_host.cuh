@@ -81,16 +81,13 @@ static int red_tables(Solver* S) {
   const int n = P.n, g1 = P.gstart[1], nB = n - g1, KC = S->sc_KC, G = P.G;
   const int nt = resident_count(S, blocks);
   if ((size_t)KC * nB > (size_t)INT32_MAX || (size_t)S->K * n > (size_t)INT32_MAX) return CMS_OK;
-  std::vector<int> ccol, tile_of, loc(nB), nb(nt, 0), tptr(nt + 1, 0), trow(nB), ttile(nB);
+  std::vector<int> ccol, tile_of, loc(nB), nb(nt, 0), tptr(nt + 1, 0), trow(nB);
   std::vector<signed char> cnt;
   CHK(schur_host_pattern(S, ccol, cnt));
   resident_partition(P, nt, tile_of);
   for (int i = 0; i < nB; ++i) loc[i] = nb[tile_of[i]]++;
   for (int t = 0; t < nt; ++t) tptr[t + 1] = tptr[t] + nb[t];
-  for (int i = 0; i < nB; ++i) {
-    trow[tptr[tile_of[i]] + loc[i]] = i;
-    ttile[tptr[tile_of[i]] + loc[i]] = tile_of[i];
-  }
+  for (int i = 0; i < nB; ++i) trow[tptr[tile_of[i]] + loc[i]] = i;
   // couplings among B rows (special rows), by side
   auto lower = [&](int i, auto&& f) {
     const int r = g1 + i;
@@ -116,6 +113,12 @@ static int red_tables(Solver* S) {
   std::vector<int> group(nB);
   for (int g = 1; g < G; ++g)
     for (int r = P.gstart[g]; r < P.gstart[g + 1]; ++r) group[r - g1] = g;
+  std::vector<int> slist, sgroup;
+  for (int g = 2; g < G; ++g) {
+    sgroup.push_back((int)slist.size());
+    for (int r = P.gstart[g]; r < P.gstart[g + 1]; ++r) slist.push_back(r);
+  }
+  sgroup.push_back((int)slist.size());
   // per tile: rows whose z (bit 2) or y (bit 1) it needs
   const int nphase = (G - 2) + (G - 1);
   std::vector<std::vector<int>> halo(nt);
@@ -260,7 +263,6 @@ static int red_tables(Solver* S) {
   };
   CHK(put(&R.tptr, tptr));
   CHK(put(&R.trow, trow));
-  CHK(put(&R.ttile, ttile));
   CHK(put(&R.tpad, tpad));
   CHK(put(&R.rexp, rexp));
   CHK(put(&R.kind, kind));
@@ -271,6 +273,8 @@ static int red_tables(Solver* S) {
   CHK(put(&R.mbase, mbase));
   CHK(put(&R.plcol, plcol));
   CHK(put(&R.ppos, ppos));
+  CHK(put(&R.slist, slist));
+  R.sgroup = sgroup;
   CHK(put(&R.spp, spp));
   CHK(put(&R.sprow, sprow));
   CHK(put(&R.spe, spe));
@@ -391,11 +395,25 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   size_t smem = 0;
   if (!red_plan<T>(R, nvec, R.limit, &nvs, &mat, &smem)) return 1;
   const double s = sizeof(T);
-  KLAUNCH(S, P_SCHUR_BUILD, (s + 4) * (double)P.nnz_off + 10.0 * n + 8.0 * (double)S->sc_nnz + s * 32.0 * 2 * R.pairs,
-          (k_red_pack<T><<<gsz(nB), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->sc_KC, R.tiles, R.tptr, R.trow, R.slptr,
-                                                         R.sloff, R.mbase, R.ttile, S->d_col, S->d_nlo, S->d_nup,
-                                                         A.aoff, A.diag, S->d_sccol, S->d_sccnt, (P2*)B.coef,
-                                                         (T*)B.cdiag)));
+  int rc = CMS_OK;
+  with_couplings(S->sc_KS, [&](auto ks) {
+    rc = [&]() -> int {
+      KLAUNCH(S, P_SCHUR_BUILD, (2 * s + 12) * (double)P.nnz_off + 10.0 * n + s * 32.0 * 2 * R.pairs,
+              (k_red_pack<T, decltype(ks)::value><<<gsz(nB), TPB, 0, S->stream>>>(
+                  n, g1, nB, P.KL, S->d_col, S->d_nlo, S->d_nup, A.aoff, A.diag, SchurMap{S->d_smap, S->d_dmap},
+                  S->d_sccnt, R.ppos, (P2*)B.coef, (T*)B.cdiag, A.luoff, A.invd)));
+      return CMS_OK;
+    }();
+  });
+  CHK(rc);
+  for (size_t g = 0; g + 1 < R.sgroup.size(); ++g) {
+    const int cnt = R.sgroup[g + 1] - R.sgroup[g];
+    if (cnt <= 0) continue;
+    KLAUNCH(S, P_ILU0, (double)cnt * 20 * s,
+            (k_red_special<T><<<gsz(cnt), TPB, 0, S->stream>>>(n, g1, P.KL, cnt, R.slist + R.sgroup[g], S->d_col,
+                                                               S->d_nlo, S->d_nup, (const T*)B.cdiag, A.luoff,
+                                                               A.invd)));
+  }
   RedArgs<T> a;
   std::memset(&a, 0, sizeof(a));
   a.n = n; a.g1 = g1; a.nB = nB; a.KL = P.KL; a.nt = a.ntiles = R.tiles;

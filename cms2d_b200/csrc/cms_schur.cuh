@@ -104,91 +104,135 @@ struct SchurArgs {
   unsigned int tag0;
 };
 
+// Tables of Chat's numeric kernels (built once per handle): for coupling c of
+// a B row (lower slots, then upper), smap[c][i] holds 8 slot bytes: a group-0
+// neighbour j's upper entries t -> the slot of row i's Chat that the product
+// with them goes to (SMAP_DIAG: the row itself, SMAP_NONE: no entry); a B
+// neighbour: its slot in byte 0.  dmap[i]: byte c is the upper entry of
+// neighbour c that leads back to the row (SMAP_NONE for B neighbours).
+constexpr int SMAP_DIAG = 0xfe, SMAP_NONE = 0xff;
+struct SchurMap {
+  const unsigned long long* smap;  // [most couplings of a B row][nB]
+  const unsigned long long* dmap;  // [nB]
+};
+
 // sinv: 1/d_r for group-0 rows, 1/s_r for B rows with
 // s_r = d_r - sum_{j in group 0} a_rj a_jr / d_j (A's off-diagonals are
-// -aoff; products accumulated in FP64).
-__global__ void __launch_bounds__(TPB) k_schur_diag(int n, int g1, int KL, const int* __restrict__ col,
+// -aoff; products accumulated in FP64).  KS: most couplings of a B row.  With
+// the table a row's loads take two round trips (the entries' search that this
+// replaces: one per entry; 1M cells 39 us, 30k 14.5 us).
+template <int KS>
+__global__ void __launch_bounds__(TPB) k_schur_diag(int n, int g1, int nB, int KL, const int* __restrict__ col,
                                                     const signed char* __restrict__ nlo,
-                                                    const signed char* __restrict__ nup,
                                                     const float* __restrict__ aoff, const float* __restrict__ diag,
-                                                    float* __restrict__ sinv) {
+                                                    SchurMap M, float* __restrict__ sinv) {
   for (int r = blockIdx.x * TPB + threadIdx.x; r < n; r += gridDim.x * TPB) {
     const float dr = diag[r];
     if (r < g1) {
       sinv[r] = 1.0f / dr;
       continue;
     }
-    double c = dr;
     const int kl = nlo[r];
-    for (int s = 0; s < kl; ++s) {
-      const size_t e = (size_t)s * n + r;
-      const int j = col[e];
-      if (j >= g1) continue;
-      const int nuj = nup[j];
-      for (int t2 = 0; t2 < nuj; ++t2) {
-        const size_t e2 = (size_t)(KL + t2) * n + j;
-        if (col[e2] == r) c -= (double)aoff[e] * (double)aoff[e2] / (double)diag[j];
+    const unsigned long long m = __ldg(M.dmap + (r - g1));
+    float a[KS], b[KS], d[KS];
+#pragma unroll
+    for (int c = 0; c < KS; ++c) {
+      const int t = (int)(m >> (8 * c)) & 0xff;
+      a[c] = 0.0f;
+      if (c < kl && t != SMAP_NONE) {
+        const size_t e = (size_t)c * n + r;
+        const int j = col[e];
+        a[c] = aoff[e];
+        b[c] = aoff[(size_t)(KL + t) * n + j];
+        d[c] = diag[j];
       }
     }
-    sinv[r] = (float)(1.0 / c);
+    double s = dr;
+#pragma unroll
+    for (int c = 0; c < KS; ++c) {
+      const int t = (int)(m >> (8 * c)) & 0xff;
+      if (c < kl && t != SMAP_NONE) s -= (double)a[c] * (double)b[c] / (double)d[c];
+    }
+    sinv[r] = (float)(1.0 / s);
+  }
+}
+
+// acc[q] (stride TPB) += the Schur complement's off-diagonals of B row r, and
+// d -= its diagonal's products:  C_rk = a_rk - sum_j a_rj a_jk / d_j.
+template <typename T, int KS>
+__device__ __forceinline__ void schur_row(int n, int g1, int nB, int KL, int i, int kl, int kt, const int* col,
+                                          const T* aoff, const T* diag, const unsigned long long* smap, double* acc,
+                                          double& d) {
+  const int r = g1 + i;
+  int j[KS];
+  T a[KS], dj[KS];
+  unsigned long long m[KS];
+#pragma unroll
+  for (int c = 0; c < KS; ++c) {
+    if (c < kt) {
+      const size_t e = (size_t)(c < kl ? c : KL + (c - kl)) * n + r;
+      j[c] = __ldg(col + e);
+      a[c] = __ldg(aoff + e);
+      m[c] = __ldg(smap + (size_t)c * nB + i);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < KS; ++c)
+    if (c < kt && j[c] < g1) dj[c] = __ldg(diag + j[c]);
+#pragma unroll
+  for (int c = 0; c < KS; ++c) {
+    if (c < kt) {
+      if (j[c] >= g1) {
+        acc[(int)(m[c] & 0xff) * TPB] += (double)a[c];
+      } else {
+        T b[KS];
+#pragma unroll
+        for (int t = 0; t < KS; ++t) {
+          b[t] = T(0);
+          if (((int)(m[c] >> (8 * t)) & 0xff) != SMAP_NONE) b[t] = __ldg(aoff + (size_t)(KL + t) * n + j[c]);
+        }
+        const double w = (double)a[c] / (double)dj[c];
+#pragma unroll
+        for (int t = 0; t < KS; ++t) {
+          const int q = (int)(m[c] >> (8 * t)) & 0xff;
+          if (q == SMAP_NONE) continue;
+          if (q == SMAP_DIAG) d -= w * (double)b[t];
+          else acc[q * TPB] += w * (double)b[t];
+        }
+      }
+    }
   }
 }
 
 // Chat's off-diagonals of reduced row i (r = g1 + i):
 // coff_rk = (aoff_rk [k in B] + sum_{j in group 0} aoff_rj aoff_jk / d_j) / s_k.
-// A thread's columns and FP64 accumulators live in shared memory, so four
-// blocks fit on an SM (with them in registers the kernel took 110 registers
-// and two blocks; its chains of dependent gathers need the extra warps).
+// A thread's FP64 accumulators live in shared memory.
+template <int KS>
 __global__ void __launch_bounds__(TPB, 4) k_schur_off(int n, int g1, int nB, int KL, int KC,
                                                    const int* __restrict__ col, const signed char* __restrict__ nlo,
                                                    const signed char* __restrict__ nup,
                                                    const float* __restrict__ aoff, const float* __restrict__ diag,
-                                                   const float* __restrict__ sinv, const int* __restrict__ ccol,
-                                                   const signed char* __restrict__ ccnt, float* __restrict__ coff,
-                                                   const int2* __restrict__ ppos, float2* __restrict__ pcoef) {
-  __shared__ double s_acc[KSC][TPB];  // this thread's columns and accumulators: column threadIdx.x
-  __shared__ int s_cc[KSC][TPB];
+                                                   SchurMap M, const float* __restrict__ sinv,
+                                                   const int* __restrict__ ccol, const signed char* __restrict__ ccnt,
+                                                   float* __restrict__ coff, const int2* __restrict__ ppos,
+                                                   float2* __restrict__ pcoef) {
+  __shared__ double s_acc[KSC][TPB];
   double* acc = &s_acc[0][threadIdx.x];
-  int* cc = &s_cc[0][threadIdx.x];
   for (int i = blockIdx.x * TPB + threadIdx.x; i < nB; i += gridDim.x * TPB) {
-    const int r = g1 + i;
-    const int kc = ccnt[i];
-    for (int q = 0; q < kc; ++q) {
-      cc[q * TPB] = ccol[(size_t)q * nB + i];
-      acc[q * TPB] = 0.0;
-    }
-    auto add = [&](int k, double v) {  // a row's columns are distinct
-      for (int q = 0; q < kc; ++q)
-        if (cc[q * TPB] == k) {
-          acc[q * TPB] += v;
-          break;
-        }
-    };
-    const int kl = nlo[r], ku = nup[r];
-    for (int s = 0; s < kl + ku; ++s) {
-      const size_t e = (size_t)(s < kl ? s : KL + (s - kl)) * n + r;
-      const int k = col[e];
-      const double a = aoff[e];
-      if (k >= g1) {
-        add(k, a);
-        continue;
+    const int kc = ccnt[i], kl = nlo[g1 + i], kt = kl + nup[g1 + i];
+    for (int q = 0; q < kc; ++q) acc[q * TPB] = 0.0;
+    double d = 0.0;
+    schur_row<float, KS>(n, g1, nB, KL, i, kl, kt, col, aoff, diag, M.smap, acc, d);
+    float prev = 0.0f;
+    const int2 pp = pcoef ? ppos[i] : make_int2(0, 0);  // the packed slices too (cms_schur_stream.cuh)
+    for (int q = 0; q < KC; ++q) {
+      const float v = q < kc ? (float)(acc[q * TPB] * (double)sinv[ccol[(size_t)q * nB + i]]) : 0.0f;
+      coff[(size_t)q * nB + i] = v;
+      if (pcoef && (q >> 1) < pp.y) {
+        if (q & 1) pcoef[(size_t)pp.x + (size_t)(q >> 1) * 32] = make_float2(prev, v);
+        else if (q + 1 == KC) pcoef[(size_t)pp.x + (size_t)(q >> 1) * 32] = make_float2(v, 0.0f);
       }
-      const double w = a / (double)diag[k];  // k is a group-0 row j
-      const int nuj = nup[k];
-      for (int t2 = 0; t2 < nuj; ++t2) {
-        const size_t e2 = (size_t)(KL + t2) * n + k;
-        const int k2 = col[e2];
-        if (k2 != r) add(k2, w * (double)aoff[e2]);
-      }
-    }
-    for (int q = 0; q < KC; ++q)
-      coff[(size_t)q * nB + i] = q < kc ? (float)(acc[q * TPB] * (double)sinv[cc[q * TPB]]) : 0.0f;
-    if (pcoef) {  // the packed slices too (cms_schur_stream.cuh): first pair and number of pairs
-      const int2 pp = ppos[i];
-      for (int q = 0; q < pp.y; ++q)
-        pcoef[(size_t)pp.x + (size_t)q * 32] =
-            make_float2(2 * q < KC ? coff[(size_t)(2 * q) * nB + i] : 0.0f,
-                        2 * q + 1 < KC ? coff[(size_t)(2 * q + 1) * nB + i] : 0.0f);
+      prev = v;
     }
   }
 }

@@ -15,6 +15,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cms_common.cuh"
@@ -69,12 +70,14 @@ struct RedTables {
   size_t words = 0, npad = 0, limit = 0;
   unsigned int tag = 1;  // first tag not used by any launch so far
   std::vector<int> hb, h_nh, h_nsp, h_ne, h_nos, h_npair;  // per tile: sizes that set the shared memory
-  int *tptr = nullptr, *trow = nullptr, *ttile = nullptr, *tpad = nullptr, *rexp = nullptr, *hptr = nullptr,
+  int *tptr = nullptr, *trow = nullptr, *tpad = nullptr, *rexp = nullptr, *hptr = nullptr,
       *hword = nullptr, *slptr = nullptr, *sloff = nullptr, *mbase = nullptr, *spp = nullptr, *spe = nullptr,
       *spoff = nullptr, *osptr = nullptr, *osrow = nullptr;
   unsigned short *kind = nullptr, *spcol = nullptr;
   int2* sprow = nullptr;
   ushort2* plcol = nullptr;
+  int* slist = nullptr;
+  std::vector<int> sgroup;  // special rows of groups >= 2 (slist): first one of each group
   int2* ppos = nullptr;  // [nB] a row's first packed pair, pairs of its slice
   ulonglong2 *xw = nullptr, *slots = nullptr;
 };
@@ -129,6 +132,8 @@ struct cms_solver {
   int *d_sccol = nullptr, *d_sdep_ptr = nullptr, *d_sdep_idx = nullptr, *d_sctr = nullptr;
   float *d_scoff = nullptr, *d_ssinv = nullptr, *d_sst = nullptr;
   signed char* d_sccnt = nullptr;
+  int sc_KS = 0;  // most couplings of a row
+  unsigned long long *d_smap = nullptr, *d_dmap = nullptr;  // SchurMap
   size_t cap_sdep = 0;
   // its resident form (cms_resident.cuh): tiles of the tables (0 none) and of
   // the last ones that did not fit, rows per thread, shared memory of the launch
@@ -728,11 +733,11 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
                         bool do_factor = true) {
   const HostPattern& P = S->hp;
   const int nb_all = S->tab.blk[S->tab.ng];
-  if (do_factor) CHK(factor<T>(S, A));
-  if (red_wanted<T>(S, 3, maxit)) {
+  if (red_wanted<T>(S, 3, maxit)) {  // (with its own part of the factor)
     const int rc = run_reduced<T>(S, A, W, 3, maxit, norm, tol, xzero);
     if (rc != 1) return rc;
   }
+  if (do_factor) CHK(factor<T>(S, A));
   if (!S->opts.multi_kernel) {
     const int tiles = persist_tiles(S);
     if (tiles > 0) {
@@ -838,11 +843,11 @@ static int run_gmres(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double tol, bo
   const HostPattern& P = S->hp;
   const int nb_all = S->tab.blk[S->tab.ng];
   const double vb = (double)P.n * sizeof(T);
-  if (do_factor) CHK(factor<T>(S, A));
   if (reduced && red_wanted<T>(S, 4, maxit)) {
     const int rc = run_reduced<T>(S, A, W, 4, maxit, 2, tol, 0);
     if (rc != 1) return rc;
   }
+  if (do_factor) CHK(factor<T>(S, A));
   if (!S->opts.multi_kernel) {
     const int rc = run_gmres_cluster<T>(S, A, W, maxit, tol);
     if (rc != 1) return rc;
@@ -976,6 +981,39 @@ static int schur_pattern(Solver* S) {
       CMS_CUDA(cudaMemcpyAsync(S->d_sctr, ctr.data(), ctr.size() * sizeof(int), cudaMemcpyHostToDevice, S->stream));
       S->sc_sym = 1;
     }
+    // where the products of the numeric kernels go (SchurMap)
+    int KS = 1, K1 = 1;  // most couplings: of any row the kernels read, of a B row
+    for (int i = 0; i < nB; ++i) K1 = std::max(K1, P.nlo[g1 + i] + P.nup[g1 + i]);
+    for (int j = 0; j < g1; ++j) KS = std::max(KS, (int)P.nup[j]);
+    KS = std::max(KS, K1);
+    if (KS > 8) return CMS_UNSUPPORTED;  // (a cell has at most 8 faces)
+    std::vector<unsigned long long> smap((size_t)K1 * nB, ~0ull), dmap(nB, ~0ull);
+    for (int i = 0; i < nB; ++i) {
+      const int r = g1 + i, kl = P.nlo[r], kt = kl + P.nup[r];
+      const int* row = &tmp[(size_t)i * KSC];
+      auto slot = [&](int k) { return (unsigned long long)(std::lower_bound(row, row + cnt[i], k) - row); };
+      auto set = [](unsigned long long& m, int b, unsigned long long v) {
+        m = (m & ~(0xffull << (8 * b))) | v << (8 * b);
+      };
+      for (int c = 0; c < kt; ++c) {
+        const int k = P.col[(size_t)(c < kl ? c : P.KL + (c - kl)) * n + r];
+        unsigned long long& m = smap[(size_t)c * nB + i];
+        if (k >= g1) {
+          set(m, 0, slot(k));
+          continue;
+        }
+        for (int t = 0; t < P.nup[k]; ++t) {
+          const int k2 = P.col[(size_t)(P.KL + t) * n + k];
+          set(m, t, k2 == r ? (unsigned long long)SMAP_DIAG : slot(k2));
+          if (k2 == r) set(dmap[i], c, (unsigned long long)t);
+        }
+      }
+    }
+    CHK(S->alloc(&S->d_smap, smap.size()));
+    CHK(S->alloc(&S->d_dmap, dmap.size()));
+    CMS_CUDA(cudaMemcpyAsync(S->d_smap, smap.data(), smap.size() * 8, cudaMemcpyHostToDevice, S->stream));
+    CMS_CUDA(cudaMemcpyAsync(S->d_dmap, dmap.data(), dmap.size() * 8, cudaMemcpyHostToDevice, S->stream));
+    S->sc_KS = KS;
     CHK(S->alloc(&S->d_sccol, ccol.size()));
     CHK(S->alloc(&S->d_scoff, ccol.size()));
     CHK(S->alloc(&S->d_sccnt, (size_t)nB));
@@ -1271,19 +1309,35 @@ static int resident_tables(Solver* S, int tiles) {
 }
 
 // Chat's values and sinv from the FP32 matrix (once per solve).
+// f(template argument) for the row kernels' bound on couplings.
+template <typename F>
+static void with_couplings(int ks, F&& f) {
+  if (ks <= 4) f(std::integral_constant<int, 4>{});
+  else if (ks <= 6) f(std::integral_constant<int, 6>{});
+  else f(std::integral_constant<int, 8>{});
+}
+
 static int schur_numeric(Solver* S, bool packed = false) {
   const HostPattern& P = S->hp;
   const int n = P.n, g1 = P.gstart[1], nB = n - g1;
   const double nnz = (double)P.nnz_off;
-  KLAUNCH(S, P_SCHUR_BUILD, 8.0 * nnz + 10.0 * n,
-          (k_schur_diag<<<gsz(n), TPB, 0, S->stream>>>(n, g1, P.KL, S->d_col, S->d_nlo, S->d_nup, S->A32.aoff,
-                                                         S->A32.diag, S->d_ssinv)));
-  KLAUNCH(S, P_SCHUR_BUILD, 8.0 * nnz + 10.0 * n + 4.0 * n + 8.0 * (double)S->sc_nnz + nB,
-          (k_schur_off<<<gsz(nB), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->sc_KC, S->d_col, S->d_nlo, S->d_nup,
-                                                        S->A32.aoff, S->A32.diag, S->d_ssinv, S->d_sccol,
-                                                        S->d_sccnt, S->d_scoff, packed ? S->rd.ppos : nullptr,
-                                                        packed ? S->st_coef : nullptr)));
-  return CMS_OK;
+  const SchurMap M{S->d_smap, S->d_dmap};
+  int rc = CMS_OK;
+  with_couplings(S->sc_KS, [&](auto ks) {
+    constexpr int KS = decltype(ks)::value;
+    rc = [&]() -> int {
+      KLAUNCH(S, P_SCHUR_BUILD, 8.0 * nnz + 18.0 * n,
+              (k_schur_diag<KS><<<gsz(n), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->d_col, S->d_nlo, S->A32.aoff,
+                                                               S->A32.diag, M, S->d_ssinv)));
+      KLAUNCH(S, P_SCHUR_BUILD, 16.0 * nnz + 10.0 * n + 4.0 * n + 8.0 * (double)S->sc_nnz + nB,
+              (k_schur_off<KS><<<gsz(nB), TPB, 0, S->stream>>>(n, g1, nB, P.KL, S->sc_KC, S->d_col, S->d_nlo, S->d_nup,
+                                                               S->A32.aoff, S->A32.diag, M, S->d_ssinv, S->d_sccol,
+                                                               S->d_sccnt, S->d_scoff, packed ? S->rd.ppos : nullptr,
+                                                               packed ? S->st_coef : nullptr)));
+      return CMS_OK;
+    }();
+  });
+  return rc;
 }
 
 // Algorithmic bytes of one reduced-system launch: the start (reduced
