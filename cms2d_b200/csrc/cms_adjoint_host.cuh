@@ -130,6 +130,7 @@ static int solve_adjoint(Solver* S, const double* acoef, const double* ss, const
   S->cur_relax = saved_relax;
   CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, st));
   CMS_CUDA(cudaStreamSynchronize(st));
+  CHK(check_waits(S));
   const DevState& h = *S->h_st;
   info->iters = h.iter;
   info->inner = h.iter;

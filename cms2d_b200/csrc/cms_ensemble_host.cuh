@@ -192,9 +192,24 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
     }
   }
   const bool inexact = schur || relax_any;
-  for (;;) {
+  // reduced form: the first residuals are normalised and solved on without
+  // waiting for their norms, and each member's correction and residual follow
+  // its inner solve on its stream, so that the host waits once per member and
+  // step while the members' kernels overlap (one wait for the residual and one
+  // for the inner solve, member after member, took a quarter of a step)
+  bool ahead = schur;
+  for (int j = 0; j < A_; ++j) ahead = ahead && refine_starts(R[j]);
+  for (bool first = true;; first = false) {
     std::vector<int> cont;
-    for (int j = 0; j < A_; ++j) {
+    if (ahead) {
+      for (int j = 0; j < A_; ++j) {
+        if (!live[j]) continue;
+        Solver* S = E->m[act[j]]->S;
+        if (first) CHK((resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, S->W64.r, nullptr, S_NRM2)));
+        cont.push_back(j);
+      }
+    }
+    for (int j = 0; j < A_ && !ahead; ++j) {
       if (!live[j]) continue;
       Solver* S = E->m[act[j]]->S;
       bool go = true, worse = false;
@@ -217,7 +232,6 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
       const int n = S->hp.n;
       KLAUNCH(S, P_VEC, (double)n * 12,
               (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
-      CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
       if (!resident)
         CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * E->tiles[i] * kProgressStride, S->stream));
       refine_inner_limits(S->opts, R[j]);
@@ -254,11 +268,19 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
     for (int j : cont) {
       Solver* S = E->m[act[j]]->S;
       CMS_CUDA(cudaStreamWaitEvent(S->stream, E->ev_done, 0));
-      CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+      if (ahead) CHK(refine_finish_step(S));
+      else
+        CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
     }
     for (int j : cont) {
       Solver* S = E->m[act[j]]->S;
       CMS_CUDA(cudaStreamSynchronize(S->stream));
+      if (ahead) {
+        bool go = false;
+        CHK(refine_outcome(S, R[j], go));
+        live[j] = go;
+        continue;
+      }
       if (S->h_st->bar.err) {
         std::snprintf(g_last_error, sizeof(g_last_error), "batched BiCGStab: a wait timed out");
         return CMS_DEVICE_ERROR;
@@ -272,13 +294,8 @@ static int refine_batched(Ens* E, const std::vector<int>& act, const std::vector
       CHK(refine_correct(S, R[j]));
     }
   }
-  for (int j = 0; j < A_; ++j) {
+  for (int j = 0; j < A_; ++j) {  // (each member's state is on the host)
     Solver* S = E->m[act[j]]->S;
-    CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
-  }
-  for (int j = 0; j < A_; ++j) {
-    Solver* S = E->m[act[j]]->S;
-    CMS_CUDA(cudaStreamSynchronize(S->stream));
     refine_finish(R[j]);
     R[j].info->rmom = S->h_st->s[S_RMOM];
   }

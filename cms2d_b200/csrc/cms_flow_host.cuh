@@ -204,8 +204,11 @@ static int solve_core64(Solver* S, int nsolv, int nswp, cms_solve_info* info, in
     // simulation would not repeat one made before
     CHK(run_krylov<double>(S, S->A64, S->W64, legacy ? 3 : nsolv, maxit, norm, tol, 0, false));
   }
-  CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
-  CMS_CUDA(cudaStreamSynchronize(S->stream));
+  if (!refine) {  // (refinement ends with the state on the host)
+    CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+    CMS_CUDA(cudaStreamSynchronize(S->stream));
+    CHK(check_waits(S));
+  }
   const DevState& h = *S->h_st;
   info->rmom = h.s[S_RMOM];
   if (plan.kind == LK_GS || plan.kind == LK_NONE) {

@@ -21,7 +21,9 @@ namespace cms {
 //   res = iwet*(sum_k acoef*phi_nb + ss - ap*phi)/ap;  rmom = sqrt(sum res^2/n)
 // and the scatter of the system into device order: diag, ELL slots, right-hand
 // side b = ss + sum over dummy neighbours of acoef*phi_dummy, x = phi.  A
-// second copy of the matrix in type TS is written when aoff2 != nullptr.
+// second copy of the matrix in type TS is written when aoff2 != nullptr.  The
+// sum of the squared residuals b - A x (before the division by ap) goes to
+// S_TRUE0: with it no pass of its own measures the initial residual.
 template <typename T, typename TS>
 __global__ void __launch_bounds__(TPB) k_prologue(int n, int nmf, const T* __restrict__ acoef, T* __restrict__ ss,
                                                   const T* __restrict__ sp, T* __restrict__ res,
@@ -32,7 +34,7 @@ __global__ void __launch_bounds__(TPB) k_prologue(int n, int nmf, const T* __res
                                                   T* __restrict__ diag, T* __restrict__ b, T* __restrict__ x,
                                                   TS* __restrict__ aoff2, TS* __restrict__ diag2,
                                                   double* partials, DevState* st) {
-  double v[1] = {0.0};
+  double v[2] = {0.0, 0.0};
   for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) {
     const T rinv = T(1) / relax;
     const T relaxm = T(1) - relax;
@@ -60,16 +62,19 @@ __global__ void __launch_bounds__(TPB) k_prologue(int n, int nmf, const T* __res
     const T ap = (sa - sp[i]) * rinv;
     const T ssi = ss[i] + relaxm * phii * ap;
     ss[i] = ssi;
-    const T resi = T(iwet[i]) * (sn + ssi - ap * phii) / ap;
+    const T num = sn + ssi - ap * phii;
+    const T resi = T(iwet[i]) * num / ap;
     res[i] = resi;
     diag[r] = ap;
     if (diag2) diag2[r] = (TS)ap;
     b[r] = ssi + gh;
     x[r] = phii;
     v[0] += (double)resi * (double)resi;
+    v[1] += (double)num * (double)num;
   }
-  if (grid_sum<1>(v, partials, &st->ticket[0])) {
+  if (grid_sum<2>(v, partials, &st->ticket[0])) {
     st->s[S_RMOM] = sqrt(v[0] / (double)n);
+    st->s[S_TRUE0] = v[1];
   }
 }
 
@@ -519,10 +524,12 @@ __global__ void __launch_bounds__(TPB) k_resid64(int n, int KL, GroupTab tab, co
   if (grid_sum(v, partials, &st->ticket[5])) st->s[slot_out] = v[0];
 }
 
-// x64 += scale * d32 (refinement correction; scale undoes the normalisation)
+// x64 += scale * d32 (refinement correction; scale undoes the normalisation),
+// unless the inner solve failed or there was nothing to correct
 __global__ void __launch_bounds__(TPB) k_ir_correct(int n, const float* __restrict__ d, double* __restrict__ x,
                                                     const DevState* st) {
   const double scale = st->s[S_IRSCALE];
+  if (st->nonfinite || st->bar.err || !(scale > 0.0)) return;
   for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) x[i] += scale * (double)d[i];
 }
 
@@ -533,13 +540,18 @@ __global__ void __launch_bounds__(TPB) k_ir_undo(int n, const float* __restrict_
   for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) x[i] -= scale * (double)d[i];
 }
 
-// r32 = r64 / ||r64||_2 (the FP32 correction solve sees a unit-norm right-hand side)
+// r32 = r64 / ||r64||_2 (the FP32 correction solve sees a unit-norm right-hand
+// side); clears the barrier of the inner solve's launch
 __global__ void __launch_bounds__(TPB) k_ir_scale(int n, const double* __restrict__ r, float* __restrict__ r32,
                                                   DevState* st) {
   const double nrm = sqrt(st->s[S_NRM2]);
   const double inv = nrm > 0.0 ? 1.0 / nrm : 0.0;
   for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) r32[i] = (float)(r[i] * inv);
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->s[S_IRSCALE] = nrm;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    st->s[S_IRSCALE] = nrm;
+    st->bar.count = st->bar.gen = 0u;
+    st->bar.err = 0;
+  }
 }
 
 template <typename TD, typename TS>

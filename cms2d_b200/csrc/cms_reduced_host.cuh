@@ -372,7 +372,9 @@ static bool red_wanted(Solver* S, int nsolv, int maxit) {
 }
 
 // The solve of A x = b (W.b, W.x) by BiCGStab (nsolv 3) or GMRES(3) (nsolv 4)
-// on the factor in A.  Returns 1 when the launch is refused.
+// on its own part of the factor.  Returns 1 when the launch is refused; does
+// not wait for the launch: the caller copies the state to the host and calls
+// check_waits.
 template <typename T>
 static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero) {
   const HostPattern& P = S->hp;
@@ -449,14 +451,10 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   S->launches++;
   const size_t nrec = S->prof_recs.size();
   prof_end(S, P_PERSIST, 0.0);
-  const bool recorded = S->prof_recs.size() > nrec;
-  CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
-  CMS_CUDA(cudaStreamSynchronize(S->stream));
-  if (S->h_st->bar.err) {
-    std::snprintf(g_last_error, sizeof(g_last_error), "reduced Krylov solve: a wait timed out");
-    return CMS_DEVICE_ERROR;
-  }
-  if (recorded) {
+  S->wait_check = true;
+  if (S->prof_recs.size() > nrec) {  // profiling: the iterations, for the byte count
+    CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+    CMS_CUDA(cudaStreamSynchronize(S->stream));
     // C's entries once per operator application; vectors: BiCGStab 26 accesses
     // of a B row per iteration, GMRES 36 per cycle
     const double C = (s + 2) * (double)S->sc_nnz;

@@ -155,6 +155,7 @@ struct cms_solver {
   float* st_vec = nullptr;
   unsigned long long* st_xnu = nullptr;
   cms::GmcPlan gmc[2];  // FP32, FP64
+  bool wait_check = false;  // a reduced Krylov launch's waits are still to be checked
   int cur_relax = 0;  // the FP32 factor in A32 is the two-phase one (k_ilu0_relax)
   int cur_fuse = 0;   // inner solves of refinement: update folded into the next iteration
   // MATRIX_SOLVER options 1, 2, 5-8: compass table (built on first use),
@@ -438,6 +439,16 @@ static int sweep_bwd(Solver* S, Mat<T>& A, Work<T>& W, T* x, int need_active) {
                                                                    A.luoff, A.invd, W.z, x, need_active, S->d_st)));
   }
   return CMS_OK;
+}
+
+// After the state's copy to the host: whether a wait of the last reduced
+// Krylov launch gave up (run_reduced does not wait for its launch).
+static int check_waits(Solver* S) {
+  if (!S->wait_check) return CMS_OK;
+  S->wait_check = false;
+  if (!S->h_st->bar.err) return CMS_OK;
+  std::snprintf(g_last_error, sizeof(g_last_error), "reduced Krylov solve: a wait timed out");
+  return CMS_DEVICE_ERROR;
 }
 
 static int poll_done(Solver* S, bool& done) {
@@ -1465,7 +1476,8 @@ static int schur_tiles(Solver* S, int layout) {
   return std::min(std::min(per * nsm, GRID_CAP), nblk(S->hp.n));
 }
 
-// The reduced FP32 inner solve (W32.b -> W32.x) as one cooperative launch.
+// The reduced FP32 inner solve (W32.b -> W32.x) as one cooperative launch,
+// after k_ir_scale (which clears its barrier).  Does not wait for it.
 enum SchurForm : int { SF_TILES = 0, SF_RESIDENT = 1, SF_STREAM = 2 };
 static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, SchurForm form) {
   const bool resident = form == SF_RESIDENT;
@@ -1473,7 +1485,6 @@ static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, Schur
   if (form == SF_STREAM) tiles = S->rd.tiles;
   SchurArgs a = make_schur_args(S, tiles, maxit, tol);
   const SchurLayout L = schur_layout(schur_layout_run(S));
-  CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   StreamArgs sa;
   size_t ssmem = 0;
   if (resident)
@@ -1499,14 +1510,11 @@ static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, Schur
   S->launches++;
   const size_t nrec = S->prof_recs.size();
   prof_end(S, P_SCHUR, 0.0);
-  const bool recorded = S->prof_recs.size() > nrec;
-  CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
-  CMS_CUDA(cudaStreamSynchronize(S->stream));
-  if (S->h_st->bar.err) {
-    std::snprintf(g_last_error, sizeof(g_last_error), "reduced BiCGStab: a grid barrier wait timed out");
-    return CMS_DEVICE_ERROR;
+  if (S->prof_recs.size() > nrec) {  // profiling: the iterations, for the byte count
+    CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+    CMS_CUDA(cudaStreamSynchronize(S->stream));
+    S->prof_recs.back().bytes = schur_bytes(S, S->h_st->iter, L.sr);
   }
-  if (recorded) S->prof_recs.back().bytes = schur_bytes(S, S->h_st->iter, L.sr);
   return CMS_OK;
 }
 
@@ -1524,17 +1532,20 @@ struct RefineState {
 // recomputed): worse = true.  BiCGStab's corrections are not monotone, so a
 // small rise is kept; a failed inner solve raises it by orders of magnitude.
 constexpr double kRefineWorse = 4.0;
-static int refine_check(Solver* S, RefineState& R, bool& go, bool& worse) {
-  const int n = S->hp.n;
-  worse = false;
+// The residual of x64 and the state, on their way to the host.
+static int refine_residual(Solver* S) {
   CHK(resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, S->W64.r, nullptr, S_NRM2));
   CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
-  CMS_CUDA(cudaStreamSynchronize(S->stream));
+  return CMS_OK;
+}
+// What follows from them once they have arrived.
+static int refine_judge(Solver* S, RefineState& R, bool& go, bool& worse) {
+  const int n = S->hp.n;
+  worse = false;
   double nrm = std::sqrt(S->h_st->s[S_NRM2]);
   if (R.steps > 0 && R.prev >= 0.0 && !(nrm <= kRefineWorse * R.prev)) {
     KLAUNCH(S, P_VEC, (double)n * 20, (k_ir_undo<<<gsz(n), TPB, 0, S->stream>>>(n, S->W32.x, S->W64.x, S->d_st)));
-    CHK(resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, S->W64.r, nullptr, S_NRM2));
-    CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
+    CHK(refine_residual(S));
     CMS_CUDA(cudaStreamSynchronize(S->stream));
     nrm = std::sqrt(S->h_st->s[S_NRM2]);
     worse = true;
@@ -1550,6 +1561,11 @@ static int refine_check(Solver* S, RefineState& R, bool& go, bool& worse) {
     go = false;
   }
   return CMS_OK;
+}
+static int refine_check(Solver* S, RefineState& R, bool& go, bool& worse) {
+  CHK(refine_residual(S));
+  CMS_CUDA(cudaStreamSynchronize(S->stream));
+  return refine_judge(S, R, go, worse);
 }
 
 // Tolerance and iteration cap of the next inner FP32 solve.  By default
@@ -1578,6 +1594,52 @@ static int refine_correct(Solver* S, RefineState& R) {
   const int n = S->hp.n;
   KLAUNCH(S, P_VEC, (double)n * 20, (k_ir_correct<<<gsz(n), TPB, 0, S->stream>>>(n, S->W32.x, S->W64.x, S->d_st)));
   ++R.steps;
+  return CMS_OK;
+}
+
+// A refinement that can start before its first residual's norm is known: the
+// first inner solve is asked for 0.5 tol of it whatever it is.
+static bool refine_starts(const RefineState& R) { return R.maxit > 0 && R.rmax > 0 && R.tol < 1.0; }
+
+// One reduced inner solve's end, enqueued behind it: the correction and the
+// residual it leaves.
+static int refine_finish_step(Solver* S) {
+  const int n = S->hp.n;
+  KLAUNCH(S, P_VEC, (double)n * 20, (k_ir_correct<<<gsz(n), TPB, 0, S->stream>>>(n, S->W32.x, S->W64.x, S->d_st)));
+  return refine_residual(S);
+}
+
+static int refine_exact(Solver* S, int nsolv, RefineState& R);
+
+// ... and its outcome, once the state has arrived: go = false ends the
+// refinement (after the exact factor's steps where the inner solve failed).
+static int refine_outcome(Solver* S, RefineState& R, bool& go) {
+  go = false;
+  if (S->h_st->bar.err) {
+    std::snprintf(g_last_error, sizeof(g_last_error), "reduced BiCGStab: a wait timed out");
+    return CMS_DEVICE_ERROR;
+  }
+  if (R.nrm0 < 0) {  // the first residual, normalised by the first step
+    R.nrm0 = R.prev = S->h_st->s[S_IRSCALE];
+    R.rel = R.nrm0 > 0 ? 1.0 : 0.0;
+    if (!std::isfinite(R.nrm0)) {
+      R.rel = R.nrm0;
+      R.info->status = CMS_NONFINITE;
+      return CMS_OK;
+    }
+    if (R.nrm0 == 0.0) return CMS_OK;
+  }
+  R.inner_total += S->h_st->iter;
+  // an FP32 inner solve that overflowed (a near-breakdown of its recurrence)
+  // gives no correction: the rest runs on the exact factor
+  if (S->h_st->nonfinite) return refine_exact(S, 3, R);
+  ++R.steps;
+  bool worse = false;
+  CHK(refine_judge(S, R, go, worse));
+  if (worse) {  // the correction was no good
+    if (go) CHK(refine_exact(S, 3, R));
+    go = false;
+  }
   return CMS_OK;
 }
 
@@ -1661,20 +1723,33 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
   R.tol = tol;
   R.maxit = maxit;
   R.rmax = S->opts.max_refine > 0 ? S->opts.max_refine : 30;
+  if (schur) {  // one wait per step: for the inner solve, its correction and the residual that leaves
+    bool go = true, worse = false;
+    if (refine_starts(R)) CHK((resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, S->W64.r, nullptr, S_NRM2)));
+    else CHK(refine_check(S, R, go, worse));
+    while (go) {
+      refine_inner_limits(S->opts, R);
+      KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
+      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, form));  // (the tiles of its layout)
+      CHK(refine_finish_step(S));
+      CMS_CUDA(cudaStreamSynchronize(S->stream));
+      CHK(refine_outcome(S, R, go));
+    }
+    refine_finish(R);
+    return CMS_OK;
+  }
   for (;;) {
     bool go = true, worse = false;
     CHK(refine_check(S, R, go, worse));
     if (worse) {  // the last inner correction was no good
-      if (go && (schur || relax)) CHK(refine_exact(S, nsolv, R));
+      if (go && relax) CHK(refine_exact(S, nsolv, R));
       break;
     }
     if (!go) break;
     // inner FP32 solve A32 d = r/||r|| from d = 0 (factor already built)
     refine_inner_limits(S->opts, R);
     KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
-    if (schur) {
-      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, form));  // tiles built above for its layout
-    } else if (nsolv == 3) {
+    if (nsolv == 3) {
       CHK(run_bicgstab<float>(S, S->A32, S->W32, R.imax, 2, R.itol, 1, false));
     } else {
       CMS_CUDA(cudaMemsetAsync(S->W32.x, 0, sizeof(float) * n, S->stream));
@@ -1684,10 +1759,10 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
     CMS_CUDA(cudaStreamSynchronize(S->stream));
     R.inner_total += (nsolv == 3) ? S->h_st->iter : S->h_st->inner;
     // an FP32 inner solve that overflowed (a near-breakdown of its recurrence)
-    // gives no correction: with the reduced or two-phase form the rest runs
-    // on the exact factor, else the refinement ends with the FP64 iterate
+    // gives no correction: with the two-phase form the rest runs on the exact
+    // factor, else the refinement ends with the FP64 iterate
     if (S->h_st->nonfinite) {
-      if (schur || relax) CHK(refine_exact(S, nsolv, R));
+      if (relax) CHK(refine_exact(S, nsolv, R));
       break;
     }
     CHK(refine_correct(S, R));
@@ -1744,13 +1819,11 @@ static int solve_dev(Solver* S, const T* acoef, T* ss, const T* sp, T* res, T* p
                                                                      relax, A.aoff, A.diag, W.b, W.x, a2, d2,
                                                                      S->d_part, S->d_st)));
   }
-  if (S->opts.verify) {
-    if (is64) CHK((resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, nullptr, nullptr, S_TRUE0)));
-    else {
-      KLAUNCH(S, P_VEC, (double)P.n * 12,
-              (k_convert<double, float><<<gsz(P.n), TPB, 0, S->stream>>>(P.n, S->W32.b, S->W64.r)));
-      CHK((resid64<float, float>(S, S->A32, S->W64.r, S->W32.x, nullptr, nullptr, S_TRUE0)));
-    }
+  const bool refine = is64 && prec == CMS_PREC_FP32_REFINE;
+  if (S->opts.verify && !is64) {  // (in FP64 the prologue measured it)
+    KLAUNCH(S, P_VEC, (double)P.n * 12,
+            (k_convert<double, float><<<gsz(P.n), TPB, 0, S->stream>>>(P.n, S->W32.b, S->W64.r)));
+    CHK((resid64<float, float>(S, S->A32, S->W64.r, S->W32.x, nullptr, nullptr, S_TRUE0)));
   }
   LegPlan plan;
   int leg_sweeps = 0;
@@ -1772,12 +1845,12 @@ static int solve_dev(Solver* S, const T* acoef, T* ss, const T* sp, T* res, T* p
     CHK(run_iccg<T>(S, A, W, maxit));
   } else if (plan.kind == LK_ICCGSTAB) {
     CHK(run_iccgstab<T>(S, A, W, maxit));
-  } else if (is64 && prec == CMS_PREC_FP32_REFINE) {
+  } else if (refine) {
     CHK(run_refine(S, legacy ? 3 : nsolv, maxit, tol, info));
   } else {
     CHK(run_krylov<T>(S, A, W, legacy ? 3 : nsolv, maxit, norm, tol, 0));
   }
-  if (S->opts.verify) {
+  if (S->opts.verify && !refine) {  // (refinement's own last residual is the same)
     if (is64) CHK((resid64<double, double>(S, S->A64, S->W64.b, S->W64.x, nullptr, nullptr, S_TRUE1)));
     else CHK((resid64<float, float>(S, S->A32, S->W64.r, S->W32.x, nullptr, nullptr, S_TRUE1)));
   }
@@ -1785,18 +1858,22 @@ static int solve_dev(Solver* S, const T* acoef, T* ss, const T* sp, T* res, T* p
           (k_scatter<T, T><<<gsz(P.n), TPB, 0, S->stream>>>(P.n, S->d_perm, W.x, phi)));
   CMS_CUDA(cudaMemcpyAsync(S->h_st, S->d_st, sizeof(DevState), cudaMemcpyDeviceToHost, S->stream));
   CMS_CUDA(cudaStreamSynchronize(S->stream));
+  CHK(check_waits(S));
   const DevState& h = *S->h_st;
   info->rmom = h.s[S_RMOM];
   if (plan.kind == LK_GS || plan.kind == LK_NONE) {
     info->iters = info->inner = leg_sweeps;  // fixed sweep count, no stopping test
-  } else if (!(is64 && prec == CMS_PREC_FP32_REFINE)) {
+  } else if (!refine) {
     info->iters = h.iter;
     info->inner = (nsolv == 4) ? h.inner : h.iter;
     info->relres = h.s[S_RELRES];
     if (h.nonfinite) info->status = CMS_NONFINITE;
     else if (!h.converged) info->status = CMS_NOT_CONVERGED;
   }
-  if (S->opts.verify) {
+  if (S->opts.verify && refine) {
+    info->true_relres = info->relres;
+    if (!std::isfinite(info->relres)) info->status = CMS_NONFINITE;
+  } else if (S->opts.verify) {
     const double t0 = std::sqrt(h.s[S_TRUE0]), t1 = std::sqrt(h.s[S_TRUE1]);
     info->true_relres = t0 > 0 ? t1 / t0 : 0.0;
     if (!std::isfinite(t1)) info->status = CMS_NONFINITE;
