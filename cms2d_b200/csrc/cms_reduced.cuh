@@ -216,7 +216,7 @@ struct RedTile {
 __device__ __forceinline__ size_t red_up16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 // Lays the tile out in shared memory and loads its tables.
-template <typename T>
+template <typename T, int BS>
 __device__ __forceinline__ void red_setup(const RedArgs<T>& A, RedTile<T>& L, unsigned char* smem, int nvec) {
   using P2 = typename Pair<T>::type;
   const int tile = A.tile;
@@ -259,16 +259,16 @@ __device__ __forceinline__ void red_setup(const RedArgs<T>& A, RedTile<T>& L, un
   if (A.mat_smem) {
     P2* cf = (P2*)take(sizeof(P2) * 32 * npair);
     ushort2* lc = (ushort2*)take(sizeof(ushort2) * 32 * npair);
-    for (int e = tid; e < npair * 32; e += RES_BS) {
+    for (int e = tid; e < npair * 32; e += BS) {
       cf[e] = __ldg(gcf + e);
       lc[e] = __ldg(glc + e);
     }
     L.cf = cf;
     L.lc = lc;
   }
-  for (int j = tid; j <= L.ns; j += RES_BS) L.soff[j] = L.ns > 0 ? __ldg(sog + j) : 0;
-  for (int k = tid; k < L.hb; k += RES_BS) L.kind[k] = k < L.nb ? __ldg(A.kind + L.t0 + k) : RED_SIMPLE;
-  for (int s = tid; s <= L.nsp; s += RES_BS) {
+  for (int j = tid; j <= L.ns; j += BS) L.soff[j] = L.ns > 0 ? __ldg(sog + j) : 0;
+  for (int k = tid; k < L.hb; k += BS) L.kind[k] = k < L.nb ? __ldg(A.kind + L.t0 + k) : RED_SIMPLE;
+  for (int s = tid; s <= L.nsp; s += BS) {
     int2 v = make_int2(0, __ldg(A.spe + s0 + s) - e0);
     if (s < L.nsp) {
       const int2 rr = __ldg(A.sprow + s0 + s);
@@ -277,11 +277,11 @@ __device__ __forceinline__ void red_setup(const RedArgs<T>& A, RedTile<T>& L, un
     }
     L.sp_row[s] = v;
   }
-  for (int e = tid; e < ne; e += RES_BS) {
+  for (int e = tid; e < ne; e += BS) {
     L.sp_val[e] = __ldg(A.luoff + __ldg(A.spoff + e0 + e));
     L.sp_col[e] = __ldg(A.spcol + e0 + e);
   }
-  for (int o = tid; o < L.nosp; o += RES_BS) {
+  for (int o = tid; o < L.nosp; o += BS) {
     const int k = __ldg(A.osrow + o0 + o);
     L.os_row[o] = (unsigned short)k;
     L.os_cd[o] = __ldg(A.cdiag + __ldg(A.trow + L.t0 + k));
@@ -291,10 +291,10 @@ __device__ __forceinline__ void red_setup(const RedArgs<T>& A, RedTile<T>& L, un
 
 // out = B part of A M^-1 (c rho, src); zb = M_S^-1 (src - c g) on own rows.
 // False when a wait gave up.
-template <typename T>
+template <typename T, int BS>
 __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>& L, const T* src, const T* g,
                                           const T* invd, double c, T* out, unsigned int tag, int zslot) {
-  constexpr int NW = RES_NW, HU = 4;
+  constexpr int NW = (BS / 32), HU = 4;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const T ct = (T)c;
   for (int j = wid; j < L.ns; j += NW) {
@@ -309,19 +309,19 @@ __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>&
   }
   bool fail = false;
   const int* hw = A.hword + __ldg(A.hptr + A.tile);
-  for (int h = threadIdx.x; h < L.nh; h += HU * RES_BS) {
+  for (int h = threadIdx.x; h < L.nh; h += HU * BS) {
     unsigned long long v[HU], t[HU];
     unsigned int spins = 0;
     int i[HU];
 #pragma unroll
-    for (int u = 0; u < HU; ++u) i[u] = __ldg(hw + (h + u * RES_BS < L.nh ? h + u * RES_BS : h));
+    for (int u = 0; u < HU; ++u) i[u] = __ldg(hw + (h + u * BS < L.nh ? h + u * BS : h));
     for (;;) {
       bool all = true;
 #pragma unroll
       for (int u = 0; u < HU; ++u) {
         v[u] = 0ull;
         t[u] = tag;
-        if (h + u * RES_BS < L.nh) ld_word16(A.xw + i[u], v[u], t[u]);
+        if (h + u * BS < L.nh) ld_word16(A.xw + i[u], v[u], t[u]);
       }
 #pragma unroll
       for (int u = 0; u < HU; ++u) all = all && t[u] == tag;
@@ -330,14 +330,14 @@ __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>&
     }
 #pragma unroll
     for (int u = 0; u < HU; ++u)
-      if (h + u * RES_BS < L.nh) from_bits(v[u], L.zb[L.hb + h + u * RES_BS]);
+      if (h + u * BS < L.nh) from_bits(v[u], L.zb[L.hb + h + u * BS]);
   }
   if (__syncthreads_or(fail)) return false;
   if (L.nsp > 0) {  // the special rows' sweeps, group by group
     const int s0 = __ldg(L.spp);
     for (int ph = 0; ph < A.nphase; ++ph) {
       const int a = __ldg(L.spp + ph) - s0, b = __ldg(L.spp + ph + 1) - s0;
-      for (int s = a + (int)threadIdx.x; s < b; s += RES_BS) {
+      for (int s = a + (int)threadIdx.x; s < b; s += BS) {
         const int2 r = L.sp_row[s];
         const int e1 = L.sp_row[s + 1].y;
         T acc = L.zb[r.x];
@@ -347,7 +347,7 @@ __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>&
       __syncthreads();
     }
     if (zslot >= 0)
-      for (int o = threadIdx.x; o < L.nosp; o += RES_BS) L.os_z[zslot * L.nosp + o] = L.zb[L.os_row[o]];
+      for (int o = threadIdx.x; o < L.nosp; o += BS) L.os_z[zslot * L.nosp + o] = L.zb[L.os_row[o]];
   }
   for (int j = wid; j < L.ns; j += NW) {
     const int k = j * 32 + lane;
@@ -369,18 +369,18 @@ __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>&
 
 // Block sums, exchanged; the totals in bc for every thread.  False on a wait
 // that gave up.
-template <typename T, int NS>
+template <typename T, int BS, int NS>
 __device__ __forceinline__ bool red_sums(const RedArgs<T>& A, const RedTile<T>& L, double (&v)[NS],
-                                         double (*sm)[RES_NW], double* bc, int buf, unsigned int tag, bool fail) {
+                                         double (*sm)[(BS / 32)], double* bc, int buf, unsigned int tag, bool fail) {
   ulonglong2* tot = A.slots + (size_t)2 * NSMAX * A.nt;
-  publish_sums<NS, RES_NW>(v, (int)(threadIdx.x >> 5) < L.ns, sm, A.slots, A.nt, A.tile, buf, tag);
-  fail |= collect_sums<NS, RES_NW>(bc, A.slots, tot, A.nt, A.tile, buf, tag, A.bar, A.spin_limit);
+  publish_sums<NS, (BS / 32)>(v, (int)(threadIdx.x >> 5) < L.ns, sm, A.slots, A.nt, A.tile, buf, tag);
+  fail |= collect_sums<NS, (BS / 32)>(bc, A.slots, tot, A.nt, A.tile, buf, tag, A.bar, A.spin_limit);
   return !__syncthreads_or(fail);
 }
 
 // Start: r = b - A x (+ add) of the own rows and this block's share of the
 // group-0 rows (stored in A.rho), g, invd, x; sums |r_B|, r_B^2, |rho|, rho^2.
-template <typename T>
+template <typename T, int BS>
 __device__ __forceinline__ bool red_start(const RedArgs<T>& A, const RedTile<T>& L, T* x, T* invd, T* g, T* r, T add,
                                           double (&s4)[4], PhaseState& ph) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n = A.n, g1 = A.g1;
@@ -401,13 +401,13 @@ __device__ __forceinline__ bool red_start(const RedArgs<T>& A, const RedTile<T>&
 #pragma unroll
   for (int q = 0; q < 4; ++q) s4[q] = 0.0;
   const int r1 = (int)((long long)g1 * (A.tile + 1) / A.nt);
-  for (int row = (int)((long long)g1 * A.tile / A.nt) + (int)threadIdx.x; row < r1; row += RES_BS) {
+  for (int row = (int)((long long)g1 * A.tile / A.nt) + (int)threadIdx.x; row < r1; row += BS) {
     const T v = resid(row, A.xzero ? T(0) : A.x[row]);
     A.rho[row] = v;
     s4[2] += fabs((double)v);
     s4[3] += (double)v * (double)v;
   }
-  for (int j = wid; j < L.ns; j += RES_NW) {
+  for (int j = wid; j < L.ns; j += (BS / 32)) {
     const int k = j * 32 + lane;
     if (k >= L.nb) continue;
     const int row = g1 + __ldg(A.trow + L.t0 + k);
@@ -421,7 +421,7 @@ __device__ __forceinline__ bool red_start(const RedArgs<T>& A, const RedTile<T>&
   }
   grid_barrier(A, ph);  // A.rho written, A.x no longer read
   if (!ph.ok) return false;
-  for (int j = wid; j < L.ns; j += RES_NW) {
+  for (int j = wid; j < L.ns; j += (BS / 32)) {
     const int k = j * 32 + lane;
     if (k >= L.nb) continue;
     const int row = g1 + __ldg(A.trow + L.t0 + k);
@@ -438,11 +438,11 @@ __device__ __forceinline__ bool red_start(const RedArgs<T>& A, const RedTile<T>&
 }
 
 // End: x_B, then x_0 = (b_0 - c rho + sub + sum aoff x_B) / d_0.
-template <typename T>
+template <typename T, int BS>
 __device__ __forceinline__ void red_finish(const RedArgs<T>& A, const RedTile<T>& L, const T* x, double c, T sub,
                                            PhaseState& ph) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int j = wid; j < L.ns; j += RES_NW) {
+  for (int j = wid; j < L.ns; j += (BS / 32)) {
     const int k = j * 32 + lane;
     if (k < L.nb) A.x[A.g1 + __ldg(A.trow + L.t0 + k)] = x[k];
   }
@@ -450,7 +450,7 @@ __device__ __forceinline__ void red_finish(const RedArgs<T>& A, const RedTile<T>
   if (!ph.ok) return;
   const T ct = (T)c;
   const int r1 = (int)((long long)A.g1 * (A.tile + 1) / A.nt);
-  for (int row = (int)((long long)A.g1 * A.tile / A.nt) + (int)threadIdx.x; row < r1; row += RES_BS) {
+  for (int row = (int)((long long)A.g1 * A.tile / A.nt) + (int)threadIdx.x; row < r1; row += BS) {
     T acc = __ldg(A.b + row) - (ct * ldm(A.rho + row) - sub);
     const int ku = __ldg(A.nup + row);
     for (int t2 = 0; t2 < ku; ++t2) {
@@ -462,12 +462,12 @@ __device__ __forceinline__ void red_finish(const RedArgs<T>& A, const RedTile<T>
 }
 
 // BiCGStab (pbicgstab.f90:20-96).
-template <typename T>
-__global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
+template <typename T, int BS>
+__global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
   extern __shared__ __align__(16) unsigned char red_smem[];
   __shared__ RedArgs<T> A;
   __shared__ RedTile<T> L;
-  __shared__ double s_sum[NSMAX][RES_NW], s_bc[NSMAX];
+  __shared__ double s_sum[NSMAX][(BS / 32)], s_bc[NSMAX];
   if (threadIdx.x == 0) {
     A = Ain;
     A.nt = A.ntiles = gridDim.x;
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
   __syncthreads();
   {
     RedTile<T> l;
-    red_setup(A, l, red_smem, RED_NV_BICG);
+    red_setup<T, BS>(A, l, red_smem, RED_NV_BICG);
     if (threadIdx.x == 0) L = l;
     __syncthreads();
   }
@@ -485,19 +485,19 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
     *r = L.vec[7];
   PhaseState ph{0u, 0u, true, true};
   auto rows = [&](auto&& f) {
-    for (int j = wid; j < ns; j += RES_NW)
+    for (int j = wid; j < ns; j += (BS / 32))
       if (j * 32 + lane < nb) f(j * 32 + lane);
   };
   unsigned int tag = A.tag0;
   int buf = 0;
   double s4[4];
-  red_start(A, L, x, invd, g, r, (T)SMALL, s4, ph);
+  red_start<T, BS>(A, L, x, invd, g, r, (T)SMALL, s4, ph);
   rows([&](int k) {
     r0[k] = r[k];
     p[k] = T(0);
     u[k] = T(0);
   });
-  bool ok = red_sums<T, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
+  bool ok = red_sums<T, BS, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
   buf ^= 1;
   const double rho1 = s_bc[2], rho2 = s_bc[3];
   double bet = s_bc[1] + rho2;
@@ -511,11 +511,11 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
     const T om = (T)omg, al = (T)alf;
     cp = cr + omg * (cp - alf * cu);
     rows([&](int k) { p[k] = r[k] + om * (p[k] - al * u[k]); });
-    ok = red_apply(A, L, p, g, invd, cp, u, tag++, -1);
+    ok = red_apply<T, BS>(A, L, p, g, invd, cp, u, tag++, -1);
     cu = cp;
     double s1[1] = {0.0};
     rows([&](int k) { s1[0] += (double)u[k] * (double)r0[k]; });
-    ok = red_sums<T, 1>(A, L, s1, s_sum, s_bc, buf, tag++, !ok);
+    ok = red_sums<T, BS, 1>(A, L, s1, s_sum, s_bc, buf, tag++, !ok);
     buf ^= 1;
     if (!ok) break;
     const double ukr0 = s_bc[0] + cu * rho2;
@@ -527,14 +527,14 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
       x[k] = x[k] + ga * L.zb[k];
       r[k] = r[k] - ga * u[k];
     });
-    ok = red_apply(A, L, r, g, invd, cr, v, tag++, -1);
+    ok = red_apply<T, BS>(A, L, r, g, invd, cr, v, tag++, -1);
     double s2[2] = {0.0, 0.0};
     rows([&](int k) {
       const double vv = v[k];
       s2[0] += vv * (double)r[k];
       s2[1] += vv * vv;
     });
-    ok = red_sums<T, 2>(A, L, s2, s_sum, s_bc, buf, tag++, !ok);
+    ok = red_sums<T, BS, 2>(A, L, s2, s_sum, s_bc, buf, tag++, !ok);
     buf ^= 1;
     if (!ok) break;
     const double vr = s_bc[0] + cr * cr * rho2, vv = fmax(s_bc[1] + cr * cr * rho2, SMALL);
@@ -550,7 +550,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
       s3[1] += (double)rn * (double)rn;
       s3[2] += (double)rn * (double)r0[k];
     });
-    ok = red_sums<T, 3>(A, L, s3, s_sum, s_bc, buf, tag++, false);
+    ok = red_sums<T, BS, 3>(A, L, s3, s_sum, s_bc, buf, tag++, false);
     buf ^= 1;
     if (!ok) break;
     const double res = A.norm == 1 ? s_bc[0] + fabs(cr) * rho1 : sqrt(s_bc[1] + cr * cr * rho2);
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_bicg(RedArgs<T> Ain) {
   }
   if (ok) {
     ph.ok = true;
-    red_finish(A, L, x, cr, (T)SMALL, ph);
+    red_finish<T, BS>(A, L, x, cr, (T)SMALL, ph);
   }
   if (A.tile == 0 && threadIdx.x == 0) {
     A.st->iter = it;
@@ -638,12 +638,12 @@ __device__ __forceinline__ bool gm_close(GmState& G, int i, double nrm2) {
   return true;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
+template <typename T, int BS>
+__global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
   extern __shared__ __align__(16) unsigned char red_smem[];
   __shared__ RedArgs<T> A;
   __shared__ RedTile<T> L;
-  __shared__ double s_sum[NSMAX][RES_NW], s_bc[NSMAX];
+  __shared__ double s_sum[NSMAX][(BS / 32)], s_bc[NSMAX];
   __shared__ GmState G;
   if (threadIdx.x == 0) {
     A = Ain;
@@ -656,7 +656,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
   __syncthreads();
   {
     RedTile<T> l;
-    red_setup(A, l, red_smem, RED_NV_GMRES);
+    red_setup<T, BS>(A, l, red_smem, RED_NV_GMRES);
     if (threadIdx.x == 0) L = l;
     __syncthreads();
   }
@@ -665,26 +665,26 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
   T *v0 = L.vec[3], *v1 = L.vec[4], *v2 = L.vec[5], *v3 = L.vec[6];
   PhaseState ph{0u, 0u, true, true};
   auto rows = [&](auto&& f) {
-    for (int j = wid; j < ns; j += RES_NW)
+    for (int j = wid; j < ns; j += (BS / 32))
       if (j * 32 + lane < nb) f(j * 32 + lane);
   };
   unsigned int tag = A.tag0;
   int buf = 0, cyc = 0;
   double s4[4];
-  red_start(A, L, x, invd, g, v0, T(0), s4, ph);
-  bool ok = red_sums<T, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
+  red_start<T, BS>(A, L, x, invd, g, v0, T(0), s4, ph);
+  bool ok = red_sums<T, BS, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
   buf ^= 1;
   const double rho2 = s_bc[3];
   while (ok && cyc < A.maxit) {
     // step 1: w = A M^-1 vh_1 (into v1); vh_1.vh_1, vh_1.w
-    ok = red_apply(A, L, v0, g, invd, G.c[0], v1, tag++, 0);
+    ok = red_apply<T, BS>(A, L, v0, g, invd, G.c[0], v1, tag++, 0);
     double a2[2] = {0.0, 0.0};
     rows([&](int k) {
       const double p = v0[k];
       a2[0] += p * p;
       a2[1] += p * (double)v1[k];
     });
-    ok = red_sums<T, 2>(A, L, a2, s_sum, s_bc, buf, tag++, !ok);
+    ok = red_sums<T, BS, 2>(A, L, a2, s_sum, s_bc, buf, tag++, !ok);
     buf ^= 1;
     if (!ok) break;
     if (threadIdx.x == 0) {
@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
       rows([&](int k) { v1[k] = p * v1[k] - q * v0[k]; });
     }
     // step 2: w = A M^-1 vh_2 (into v2)
-    ok = red_apply(A, L, v1, g, invd, G.c[1], v2, tag++, 1);
+    ok = red_apply<T, BS>(A, L, v1, g, invd, G.c[1], v2, tag++, 1);
     double b4[4] = {0.0, 0.0, 0.0, 0.0};
     rows([&](int k) {
       const double p = v0[k], q = v1[k], w = v2[k];
@@ -715,7 +715,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
       b4[2] += p * w;
       b4[3] += q * w;
     });
-    ok = red_sums<T, 4>(A, L, b4, s_sum, s_bc, buf, tag++, !ok);
+    ok = red_sums<T, BS, 4>(A, L, b4, s_sum, s_bc, buf, tag++, !ok);
     buf ^= 1;
     if (!ok) break;
     if (threadIdx.x == 0) {
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
         rows([&](int k) { v2[k] = p * v2[k] - q * v0[k] - s * v1[k]; });
       }
       // step 3: w = A M^-1 vh_3 (into v3)
-      ok = red_apply(A, L, v2, g, invd, G.c[2], v3, tag++, 2);
+      ok = red_apply<T, BS>(A, L, v2, g, invd, G.c[2], v3, tag++, 2);
       double c6[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
       rows([&](int k) {
         const double p = v0[k], q = v1[k], s = v2[k], w = v3[k];
@@ -750,7 +750,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
       });
       // (vh_2.vh_1 is needed again: kept in G.y until the cycle's end)
       if (threadIdx.x == 0) G.y[0] = s_bc[1];
-      ok = red_sums<T, 6>(A, L, c6, s_sum, s_bc, buf, tag++, !ok);
+      ok = red_sums<T, BS, 6>(A, L, c6, s_sum, s_bc, buf, tag++, !ok);
       buf ^= 1;
       if (!ok) break;
       if (threadIdx.x == 0) {
@@ -778,7 +778,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
           v3[k] = w;
           d1[0] += (double)w * (double)w;
         });
-        ok = red_sums<T, 1>(A, L, d1, s_sum, s_bc, buf, tag++, false);
+        ok = red_sums<T, BS, 1>(A, L, d1, s_sum, s_bc, buf, tag++, false);
         buf ^= 1;
         if (!ok) break;
         if (threadIdx.x == 0) gm_close(G, 2, s_bc[0] + G.c[3] * G.c[3] * rho2);
@@ -823,7 +823,7 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
   }
   if (ok) {
     ph.ok = true;
-    red_finish(A, L, x, G.c[0], T(0), ph);
+    red_finish<T, BS>(A, L, x, G.c[0], T(0), ph);
   }
   if (A.tile == 0 && threadIdx.x == 0) {
     A.st->iter = cyc;
@@ -834,6 +834,15 @@ __global__ void __launch_bounds__(RES_BS, 1) k_red_gmres(RedArgs<T> Ain) {
     A.st->nonfinite = G.nonfinite;
     A.st->done = 1;
   }
+}
+
+// The kernel for a method (3 BiCGStab, FP64 only; 4 GMRES) and block size.
+template <typename T>
+inline const void* red_kernel(int nsolv, int bs) {
+  if constexpr (sizeof(T) == 8) {
+    if (nsolv == 3) return bs == 512 ? (const void*)k_red_bicg<T, 512> : (const void*)k_red_bicg<T, 1024>;
+  }
+  return bs == 512 ? (const void*)k_red_gmres<T, 512> : (const void*)k_red_gmres<T, 1024>;
 }
 
 }  // namespace cms

@@ -5,6 +5,8 @@
 
 namespace cms {
 
+constexpr int RED_WIDE = 1024;  // rows per tile above which a block has 1024 threads
+
 // Shared memory of a tile besides its vectors and packed coefficients.
 template <typename T>
 static size_t red_smem_base(const RedTables& R, int t) {
@@ -53,8 +55,9 @@ static int stream_vectors(const RedTables& R, size_t limit, size_t* smem) {
 static int red_limit(Solver* S, size_t* limit) {
   int optin = 0;
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, S->dev) != cudaSuccess) return CMS_DEVICE_ERROR;
-  const void* k[4] = {(const void*)k_red_bicg<double>, (const void*)k_red_gmres<double>,
-                      (const void*)k_red_gmres<float>, (const void*)k_schur_stream};
+  const void* k[7] = {red_kernel<double>(3, 512), red_kernel<double>(3, 1024), red_kernel<double>(4, 512),
+                      red_kernel<double>(4, 1024), red_kernel<float>(4, 512), red_kernel<float>(4, 1024),
+                      (const void*)k_schur_stream};
   size_t most = (size_t)optin;
   for (const void* f : k) {
     cudaFuncAttributes fa;
@@ -358,11 +361,12 @@ static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
 // k_bicg_persistent; so do refinement's inner solves with inner_relax 0 or 1.
 // Solve times, one B200 (per-phase kernels for GMRES, k_bicg_persistent for
 // BiCGStab / reduced form):
-//   GMRES(3) to 1e-3     20k cells 1.29 / 0.27 ms, 1M 4.39 / 0.95, 4M 10.9 / 4.5
-//   BiCGStab to 1e-6     100k cells 1.7 / 0.56 ms, 1M 4.9 / 1.5, 4M 14.0 / 8.4
+//   GMRES(3) to 1e-3     20k cells 1.29 / 0.21 ms, 1M 4.39 / 0.75, 4M 10.7 / 2.8
+//   BiCGStab to 1e-6     100k cells 1.7 / 0.50 ms, 1M 4.9 / 1.13, 4M 14.0 / 5.3
 // What bounds it: up to 250k cells the exchanges and sums (2 and 3 per
 // BiCGStab iteration, 3 and 4 per GMRES cycle), at 1M the coefficients read
-// from L2 (40 MB per application), at 4M HBM latency at 16 warps per SM.
+// from L2 (40 MB per application), at 4M HBM (160 MB per application and the
+// vectors).
 template <typename T>
 static bool red_wanted(Solver* S, int nsolv, int maxit) {
   if (S->opts.multi_kernel || S->opts.ordering != CMS_ORDER_MULTICOLOR || S->cur_relax || S->cur_fuse || maxit < 1 ||
@@ -434,11 +438,13 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   void* args[] = {&a};
   prof_begin(S);
-  const void* kern = (const void*)k_red_gmres<T>;
-  if constexpr (sizeof(T) == 8) {
-    if (nsolv == 3) kern = (const void*)k_red_bicg<T>;
-  }
-  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(R.tiles), dim3(RES_BS), args, smem, S->stream);
+  // 1024 threads where a tile has more rows than that, for the loads in flight
+  // (BiCGStab at 1M cells, 3400 rows: 1330 us with 512, 1129 with 1024; GMRES at
+  // 4M 4.46 and 2.81 ms); below, fewer warps make the sums shorter (gradient at
+  // 100k cells, 340 rows: 1611 and 1815 us)
+  const int bs = *std::max_element(R.hb.begin(), R.hb.end()) > RED_WIDE ? 1024 : 512;
+  const void* kern = red_kernel<T>(nsolv, bs);
+  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(R.tiles), dim3(bs), args, smem, S->stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
     R.state = -1;
