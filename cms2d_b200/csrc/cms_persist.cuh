@@ -205,6 +205,56 @@ __device__ __forceinline__ void get_totals(const Args& A, double (&tot)[NS], int
   __syncthreads();
 }
 
+// This block's partial sums of NS values into buffer buf: warp sums in
+// shared memory, then warp q adds value q over the block's warps (fixed
+// order) and its lane 0 stores it.  The stores are ordered before the
+// phase's progress release by end_phase's __syncthreads.
+template <int NS, int BS, class Args>
+__device__ __forceinline__ void put_partials_bs(const Args& A, double (&v)[NS], int buf) {
+  constexpr int NW = BS / 32;
+  __shared__ double sm[NS][NW];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < NS; ++q) v[q] = warp_sum(v[q]);
+  if (lane == 0) {
+#pragma unroll
+    for (int q = 0; q < NS; ++q) sm[q][wid] = v[q];
+  }
+  __syncthreads();
+  for (int q = wid; q < NS; q += NW) {
+    const double x = warp_sum(lane < NW ? sm[q][lane] : 0.0);
+    if (lane == 0) A.part[((size_t)buf * NSMAX + q) * A.ntiles + A.tile] = x;
+  }
+}
+
+// After a grid barrier: the grid totals, value q summed by warp q (lane l
+// adds tiles l, l + 32, ... in that order, then a butterfly), so every block
+// forms the same bits; then shared with the block.  A lane's loads for up
+// to 256 tiles are issued before their adds (one round trip; the missing ones
+// add 0, which changes no bits).
+template <int NS, int BS, class Args>
+__device__ __forceinline__ void get_totals_w0(const Args& A, double (&tot)[NS], int buf) {
+  constexpr int NW = BS / 32;
+  __shared__ double bc[NS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nt = A.ntiles;
+  for (int q = wid; q < NS; q += NW) {
+    const double* src = A.part + ((size_t)buf * NSMAX + q) * nt;
+    double acc = 0.0;
+    for (int b = lane; b < nt; b += 256) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = b + 32 * u < nt ? __ldcg(src + b + 32 * u) : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) acc += v[u];
+    }
+    acc = warp_sum(acc);
+    if (lane == 0) bc[q] = acc;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NS; ++q) tot[q] = bc[q];
+}
+
 // Rows of this block's tile in group g.
 template <typename T>
 __device__ __forceinline__ int2 tile_rows(const PersistArgs<T>& A, int g) {
@@ -517,8 +567,20 @@ __device__ __forceinline__ void pc_apply(const PersistArgs<T>& A, PhaseState& ph
 }
 
 // The solve run by one block (tile A.tile of the system A describes).
-template <typename T>
+// (BS: threads per block; blocks of 256 threads add their sums as block_sum
+// does, wider ones a value per warp)
+template <typename T, int BS>
 __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
+  auto put = [&](auto& v, int buf) {
+    constexpr int NS = sizeof(v) / sizeof(double);
+    if constexpr (BS == TPB) put_partials<NS>(A, v, buf);
+    else put_partials_bs<NS, BS>(A, v, buf);
+  };
+  auto get = [&](auto& v, int buf) {
+    constexpr int NS = sizeof(v) / sizeof(double);
+    if constexpr (BS == TPB) get_totals<NS>(A, v, buf);
+    else get_totals_w0<NS, BS>(A, v, buf);
+  };
   constexpr int NR = NRT<T>;
   const int G = A.G;
   PhaseState ph{0u, 0u, true, true};
@@ -572,11 +634,11 @@ __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
         }
       });
     }
-    put_partials<2>(A, s2, 0);
+    put(s2, 0);
     end_phase(A, ph);
     grid_barrier(A, ph);
     if (ph.ok) {
-      get_totals<2>(A, s2, 0);
+      get(s2, 0);
       res0 = (A.norm == 1) ? s2[0] : sqrt(s2[1]);
       bet = s2[1];
     }
@@ -611,11 +673,11 @@ __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
           }
         });
       }
-      put_partials<1>(A, s1, buf);
+      put(s1, buf);
       end_phase(A, ph);
       grid_barrier(A, ph);
       if (!ph.ok) break;
-      get_totals<1>(A, s1, buf);
+      get(s1, buf);
       buf ^= 1;
       gam = bet / s1[0];
       bet0 = bet;
@@ -648,18 +710,18 @@ __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
           }
         });
       }
-      if (A.fuse_upd) put_partials<5>(A, s5, buf);
+      if (A.fuse_upd) put(s5, buf);
       else {
         double s2[2] = {s5[0], s5[1]};
-        put_partials<2>(A, s2, buf);
+        put(s2, buf);
       }
       end_phase(A, ph);
       grid_barrier(A, ph);
       if (!ph.ok) break;
-      if (A.fuse_upd) get_totals<5>(A, s5, buf);
+      if (A.fuse_upd) get(s5, buf);
       else {
         double s2[2];
-        get_totals<2>(A, s2, buf);
+        get(s2, buf);
         s5[0] = s2[0]; s5[1] = s2[1];
       }
       buf ^= 1;
@@ -699,11 +761,11 @@ __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
           }
         });
       }
-      put_partials<3>(A, s3, buf);
+      put(s3, buf);
       end_phase(A, ph);
       grid_barrier(A, ph);
       if (!ph.ok) break;
-      get_totals<3>(A, s3, buf);
+      get(s3, buf);
       buf ^= 1;
       const double res = (A.norm == 1) ? s3[0] : sqrt(s3[1]);
       rel = res / res0;
@@ -743,8 +805,8 @@ __device__ __forceinline__ void bicg_body(const PersistArgs<T>& A) {
 }
 
 // One system: block b works on tile b.
-template <typename T>
-__global__ void __launch_bounds__(TPB, 4) k_bicg_persistent(PersistArgs<T> A) {
+template <typename T, int BS = TPB>
+__global__ void __launch_bounds__(BS, 1024 / BS) k_bicg_persistent(PersistArgs<T> A) {
   __shared__ PersistArgs<T> sA;
   if (threadIdx.x == 0) {
     sA = A;
@@ -752,7 +814,7 @@ __global__ void __launch_bounds__(TPB, 4) k_bicg_persistent(PersistArgs<T> A) {
     sA.tile = blockIdx.x;
   }
   __syncthreads();
-  bicg_body<T>(sA);
+  bicg_body<T, BS>(sA);
 }
 
 // Several independent systems (an ensemble) in one launch: bmap[b] = (member,
@@ -769,7 +831,7 @@ __global__ void __launch_bounds__(TPB, 4) k_bicg_batched(const PersistArgs<T>* _
     sA.tile = mt.y;
   }
   __syncthreads();
-  bicg_body<T>(sA);
+  bicg_body<T, TPB>(sA);
 }
 
 // Failure-detection check of the waits above: one block runs tile 0 of a

@@ -237,56 +237,6 @@ __global__ void __launch_bounds__(TPB, 4) k_schur_off(int n, int g1, int nB, int
   }
 }
 
-// This block's partial sums of NS values into buffer buf: warp sums in
-// shared memory, then warp q adds value q over the block's warps (fixed
-// order) and its lane 0 stores it.  The stores are ordered before the
-// phase's progress release by end_phase's __syncthreads.
-template <int NS, int BS>
-__device__ __forceinline__ void put_partials_bs(const SchurArgs& A, double (&v)[NS], int buf) {
-  constexpr int NW = BS / 32;
-  __shared__ double sm[NS][NW];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NS; ++q) v[q] = warp_sum(v[q]);
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < NS; ++q) sm[q][wid] = v[q];
-  }
-  __syncthreads();
-  for (int q = wid; q < NS; q += NW) {
-    const double x = warp_sum(lane < NW ? sm[q][lane] : 0.0);
-    if (lane == 0) A.part[((size_t)buf * NSMAX + q) * A.ntiles + A.tile] = x;
-  }
-}
-
-// After a grid barrier: the grid totals, value q summed by warp q (lane l
-// adds tiles l, l + 32, ... in that order, then a butterfly), so every block
-// forms the same bits; then shared with the block.  A lane's loads for up
-// to 256 tiles are issued before their adds (one round trip; the missing ones
-// add 0, which changes no bits).
-template <int NS, int BS>
-__device__ __forceinline__ void get_totals_w0(const SchurArgs& A, double (&tot)[NS], int buf) {
-  constexpr int NW = BS / 32;
-  __shared__ double bc[NS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nt = A.ntiles;
-  for (int q = wid; q < NS; q += NW) {
-    const double* src = A.part + ((size_t)buf * NSMAX + q) * nt;
-    double acc = 0.0;
-    for (int b = lane; b < nt; b += 256) {
-      double v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = b + 32 * u < nt ? __ldcg(src + b + 32 * u) : 0.0;
-#pragma unroll
-      for (int u = 0; u < 8; ++u) acc += v[u];
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) bc[q] = acc;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NS; ++q) tot[q] = bc[q];
-}
-
 // Rows of this tile in groups ga..gb as one index space (ranges in shared
 // memory: s_lo first row of each group's range, s_pre prefix counts).
 template <int NR, typename F>

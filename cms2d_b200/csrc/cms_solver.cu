@@ -121,6 +121,7 @@ struct cms_solver {
   int *d_toff = nullptr, *d_dep_ptr = nullptr, *d_dep_idx = nullptr;
   unsigned int* d_progress = nullptr;
   double* d_ppart = nullptr;
+  bool tiles_set = false;  // their number was set by the caller
   int ptiles = 0;  // tiles (= blocks) of the persistent kernel; 0 not built, -1 not launchable
   size_t cap_toff = 0, cap_dep = 0;  // capacities of d_toff / d_dep_idx
   // reduced (Schur complement) inner solve of refinement (cms_schur.cuh):
@@ -586,6 +587,25 @@ static int build_tiles(Solver* S, int nt) {
   return nt;
 }
 
+// FP32 systems of more than 1024 rows per SM run as one block of 1024 threads
+// per SM instead of four of 256: a quarter of the blocks arrive at a barrier and
+// leave partial sums, and fewer tiles wait on each other (solve to 1e-5, same
+// bits: 152k cells 1728 -> 1533 us, 1M 2944 -> 2639 us telescoping; 1200 ->
+// 1008 us and 1919 -> 1798 us Cartesian).
+// Builds the tiles; not when cms_solver_set_tiles chose their number.
+template <typename T>
+static bool persist_wide(Solver* S) {
+  if (sizeof(T) != 4 || S->tiles_set || S->hp.G > GFLAT) return false;
+  int nsm = 0, per = 0;
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, S->dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bicg_persistent<float, 1024>, 1024, 0) != cudaSuccess ||
+      per < 1) {
+    cudaGetLastError();
+    return false;
+  }
+  return S->hp.n > nsm * 1024 && persist_tiles(S) > 0 && build_tiles(S, nsm) == nsm;
+}
+
 // Algorithmic bytes of one persistent launch (each array a phase touches
 // counted once per phase): the start, then per iteration two preconditioner
 // applications (forward phases with their right-hand side formed in place,
@@ -702,14 +722,17 @@ static int persist_wait_selftest(Solver* S, unsigned int spin_limit, int which) 
 // caller can fall back to the per-phase kernels.
 template <typename T>
 static int run_bicgstab_persistent(Solver* S, Mat<T>& A, Work<T>& W, int tiles, int maxit, int norm, double tol,
-                                   int xzero) {
+                                   int xzero, bool wide) {
   PersistArgs<T> a = make_args<T>(S, A, W, tiles, maxit, norm, tol, xzero);
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
   void* args[] = {&a};
   prof_begin(S);
-  const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_bicg_persistent<T>, dim3(tiles), dim3(TPB), args,
-                                                    0, S->stream);
+  const void* kern = (const void*)k_bicg_persistent<T>;
+  if constexpr (sizeof(T) == 4) {
+    if (wide) kern = (const void*)k_bicg_persistent<T, 1024>;
+  }
+  const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(tiles), dim3(wide ? 1024 : TPB), args, 0, S->stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
     S->ptiles = -1;
@@ -750,9 +773,10 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
   }
   if (do_factor) CHK(factor<T>(S, A));
   if (!S->opts.multi_kernel) {
+    const bool wide = persist_wide<T>(S);
     const int tiles = persist_tiles(S);
     if (tiles > 0) {
-      const int rc = run_bicgstab_persistent<T>(S, A, W, tiles, maxit, norm, tol, xzero);
+      const int rc = run_bicgstab_persistent<T>(S, A, W, tiles, maxit, norm, tol, xzero, wide);
       if (rc != 1) return rc;
     }
   }
@@ -1945,6 +1969,7 @@ int cms_solver_set_tiles(cms_solver* s, int tiles) {
   if (!s || tiles < 0) return -CMS_BAD_ARGUMENT;
   const int cap = cms::persist_capacity(s->dev);
   if (cap <= 0) return -CMS_UNSUPPORTED;
+  s->tiles_set = tiles > 0;
   const int nt = cms::build_tiles(s, tiles == 0 ? std::min(cap, cms::nblk(s->hp.n)) : std::min(tiles, cap));
   return nt > 0 ? nt : -CMS_UNSUPPORTED;
 }
