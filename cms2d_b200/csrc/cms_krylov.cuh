@@ -495,7 +495,11 @@ __global__ void k_gm_start(DevState* st, int maxit, double tol) {
 
 // ----------------------------------------------------------------------------
 // FP64 residual of the device-order system, r = b - A x (all rows), sum r^2
-// into S_NRM2 (slot_out).  Optionally stores r (FP64) and its FP32 copy.
+// into S_NRM2 (slot_out).  Optionally stores r (FP64) and its FP32 copy.  A
+// row's couplings (at most 8: a cell has at most 8 faces) are loaded together,
+// then the gathered values together: three dependent round trips per row
+// instead of one per coupling (30k rows 6.7 -> 4.6 us, 4M 103 -> 93 us; bound by
+// latency below and by HBM above).
 template <typename TA, typename TX>
 __global__ void __launch_bounds__(TPB) k_resid64(int n, int KL, GroupTab tab, const int* __restrict__ col,
                                                  const signed char* __restrict__ nlo,
@@ -508,15 +512,27 @@ __global__ void __launch_bounds__(TPB) k_resid64(int n, int KL, GroupTab tab, co
   const int stride = (tab.blk[g + 1] - tab.blk[g]) * TPB;
   double v[1] = {0.0};
   for (int r = tab.start[g] + (blockIdx.x - tab.blk[g]) * TPB + threadIdx.x; r < tab.start[g + 1]; r += stride) {
-    const int kl = tab.kl[g] > 0 ? (int)nlo[r] : 0, ku = tab.ku[g] > 0 ? (int)nup[r] : 0;
+    const int kl = nlo[r], k = kl + nup[r];
+    const double br = b[r], dr = (double)diag[r], xr = (double)x[r];
+    int c[8];
+    TA a[8];
+    TX xv[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (q < k) {
+        const size_t e = (size_t)(q < kl ? q : KL + (q - kl)) * n + r;
+        c[q] = col[e];
+        a[q] = aoff[e];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (q < k) xv[q] = x[c[q]];
     double sum = 0.0;
 #pragma unroll
-    for (int s = 0; s < KMAX; ++s)
-      if (s < kl) sum += (double)aoff[(size_t)s * n + r] * (double)x[col[(size_t)s * n + r]];
-#pragma unroll
-    for (int t = 0; t < KMAX; ++t)
-      if (t < ku) sum += (double)aoff[(size_t)(KL + t) * n + r] * (double)x[col[(size_t)(KL + t) * n + r]];
-    const double rr = b[r] - ((double)diag[r] * (double)x[r] - sum);
+    for (int q = 0; q < 8; ++q)
+      if (q < k) sum += (double)a[q] * (double)xv[q];
+    const double rr = br - (dr * xr - sum);
     if (rout) rout[r] = rr;
     if (rout32) rout32[r] = (float)rr;
     v[0] += rr * rr;
