@@ -1343,7 +1343,6 @@ static int resident_tables(Solver* S, int tiles) {
   return CMS_OK;
 }
 
-// Chat's values and sinv from the FP32 matrix (once per solve).
 // f(template argument) for the row kernels' bound on couplings.
 template <typename F>
 static void with_couplings(int ks, F&& f) {
@@ -1352,6 +1351,7 @@ static void with_couplings(int ks, F&& f) {
   else f(std::integral_constant<int, 8>{});
 }
 
+// Chat's values and sinv from the FP32 matrix (once per solve).
 static int schur_numeric(Solver* S, bool packed = false) {
   const HostPattern& P = S->hp;
   const int n = P.n, g1 = P.gstart[1], nB = n - g1;
