@@ -287,6 +287,8 @@ __global__ void __launch_bounds__(GMC_BS, 1) k_gmres_cluster(GmcArgs<T> Ain) {
     }
     gmc_sync();
   };
+  // every block of the cluster has started before the first store to its shared memory (put_part)
+  gmc_sync();
   while (!G.done) {
     // restart residual v_1 = b - A x
     for (int lv = slot; lv < nlv; lv += GMC_SLOTS) {
