@@ -116,10 +116,12 @@ __device__ __forceinline__ void gmc_scalars(GmcState& G, int j, int i, double v)
 
 // Barrier of the cluster that orders all its threads' accesses: the block
 // barrier, one thread's fence, then the hardware barrier without a fence of
-// its own (every warp's fence took most of a phase).
+// its own (every warp's fence took most of a phase).  The .aligned forms want a
+// converged warp, which the fence's branch leaves open.
 __device__ __forceinline__ void gmc_sync() {
   __syncthreads();
   if (threadIdx.x == 0) asm volatile("fence.acq_rel.cluster;" ::: "memory");
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

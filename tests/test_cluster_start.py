@@ -1,7 +1,9 @@
-"""A block of a cluster may store to another block's shared memory only after that block has started, which a
-barrier of the whole cluster ensures.  A missing one shows on a GPU only when the blocks happen to start apart,
-so the order is read from the kernel's source: on every path, the barrier comes before the first of the stores
-(put_part), both outside the functions that only define them."""
+"""The order of the cluster GMRES's barriers, read from its source (none of it shows on a GPU except by chance).
+
+A block of a cluster may store to another block's shared memory only after that block has started, which a
+barrier of the whole cluster ensures: on every path it comes before the first of the stores (put_part), both
+outside the functions that only define them.  And a warp reaches an .aligned barrier converged: after a branch
+of single threads a __syncwarp or __syncthreads comes first."""
 import os
 import re
 
@@ -40,3 +42,12 @@ def test_cluster_barrier_before_first_remote_store():
     assert "map_shared_rank" not in body  # remote stores are made by put_part only
     assert barrier < first_store
     assert body[:barrier].count("{") == body[:barrier].count("}")  # not inside a branch or a loop
+
+
+def test_warps_reach_aligned_barriers_converged():
+    body = re.sub(r"//[^\n]*", "", open(SRC).read())
+    fn = body[body.index("void gmc_sync()"):]
+    fn = fn[:fn.index("\n}")]
+    assert fn.count(".aligned") == 2
+    before = fn[:fn.index("barrier.cluster.arrive")]
+    assert max(before.rfind("__syncwarp()"), before.rfind("__syncthreads()")) > before.rfind("if (")
