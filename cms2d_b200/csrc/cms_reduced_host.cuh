@@ -285,7 +285,7 @@ static int red_tables(Solver* S) {
   CHK(put(&R.spcol, spcol));
   CHK(put(&R.osptr, osptr));
   CHK(put(&R.osrow, osrow));
-  CHK(S->alloc(&R.xw, words + 1));
+  CHK(S->alloc(&R.xw, STR_ST_COPIES * (words + 1)));  // (the streamed form's copies of s, t)
   CHK(S->alloc(&R.slots, (size_t)2 * (NSMAX * nt + RES_TOT)));
   CMS_CUDA(cudaStreamSynchronize(s));
   R.words = words;
@@ -302,7 +302,7 @@ static int red_tables(Solver* S) {
 static int red_tags(Solver* S, unsigned int need, unsigned int* tag0) {
   RedTables& R = S->rd;
   if (R.tag > 0xffffffffu - need) {
-    CMS_CUDA(cudaMemsetAsync(R.xw, 0, (R.words + 1) * sizeof(ulonglong2), S->stream));
+    CMS_CUDA(cudaMemsetAsync(R.xw, 0, STR_ST_COPIES * (R.words + 1) * sizeof(ulonglong2), S->stream));
     CMS_CUDA(cudaMemsetAsync(R.slots, 0, (size_t)2 * (NSMAX * R.tiles + RES_TOT) * sizeof(ulonglong2), S->stream));
     if (S->st_xnu) CMS_CUDA(cudaMemsetAsync(S->st_xnu, 0, (R.words + 1) * sizeof(unsigned long long), S->stream));
     R.tag = 1;
@@ -349,7 +349,7 @@ static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
   const double mat = 32.0 * R.pairs * (sizeof(float2) + sizeof(ushort2)), vecs = (SV_N - a->nvs) * 4.0 * (double)R.npad;
   constexpr double kL2Keep = 75e6;
   a->keep = (float)std::min(1.0, std::max(0.0, (kL2Keep - vecs) / mat));
-  a->xst = R.xw; a->xnu = S->st_xnu; a->slots = R.slots;
+  a->xst = R.xw; a->words = R.words + 1; a->xnu = S->st_xnu; a->slots = R.slots;
   return red_tags(S, (unsigned int)maxit + 2u, &a->S.tag0);
 }
 

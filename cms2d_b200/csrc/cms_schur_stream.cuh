@@ -12,6 +12,15 @@
 // are done in the gather's loop.  About 310 MB per iteration, less what the
 // vectors kept in shared memory save (the first ones of SV_* that fit).
 //
+// Why a word is never overwritten too early.  The halo is the reduced Krylov
+// solves' one, extended along the special rows: a tile may read another's words
+// while that one reads none of its (an inlet of 2.0M cells has such a pair), so
+// the argument of cms_resident.cuh for s and t, which needs every edge both ways, does not hold.
+// s and t have STR_ST_COPIES = 2 copies by the tag's parity: those of iteration
+// i are replaced by those of i+2, after the sums of i+1, which a reader
+// contributes to after it has read s, t of i.  nu and the sums are as in
+// cms_resident.cuh, whose argument for them needs no symmetry.
+//
 // Measured: at its rule, stream_choose in cms_reduced_host.cuh.
 #pragma once
 #include "cms_reduced.cuh"
@@ -20,6 +29,7 @@ namespace cms {
 
 constexpr int STR_BS = 1024;
 constexpr int STR_NW = STR_BS / 32;
+constexpr int STR_ST_COPIES = 2;  // of the words of s and t
 // vectors in the order in which they are kept in shared memory
 enum StreamVec : int { SV_S = 0, SV_T, SV_Y, SV_P, SV_U, SV_Q, SV_R0, SV_F0, SV_N };
 
@@ -32,7 +42,8 @@ struct StreamArgs {
   size_t npad;
   int nvs;
   float keep;                // share of the slices that L2 is to keep
-  ulonglong2* xst;
+  ulonglong2* xst;           // [STR_ST_COPIES][words]
+  size_t words;
   unsigned long long* xnu;
   ulonglong2* slots;
 };
@@ -113,6 +124,7 @@ __global__ void __launch_bounds__(STR_BS, 1) k_schur_stream(StreamArgs Ain) {
   constexpr int HU = 2;
   auto halo_st = [&](unsigned int tag) -> bool {
     bool fail = false;
+    const ulonglong2* xst = B.xst + tag % STR_ST_COPIES * B.words;
     for (int h = threadIdx.x; h < nh; h += HU * STR_BS) {
       unsigned long long v[HU], t[HU];
       unsigned int spins = 0;
@@ -125,7 +137,7 @@ __global__ void __launch_bounds__(STR_BS, 1) k_schur_stream(StreamArgs Ain) {
         for (int u = 0; u < HU; ++u) {
           v[u] = 0ull;
           t[u] = tag;
-          if (h + u * STR_BS < nh) ld_word16(B.xst + i[u], v[u], t[u]);
+          if (h + u * STR_BS < nh) ld_word16(xst + i[u], v[u], t[u]);
           all = all && t[u] == tag;
         }
         if (all) break;
@@ -168,7 +180,8 @@ __global__ void __launch_bounds__(STR_BS, 1) k_schur_stream(StreamArgs Ain) {
   };
   auto put_st = [&](int k, float s, float t, unsigned int tag) {
     const int w = __ldg(rexp + k);
-    if (w >= 0) st_word16(B.xst + w, (unsigned long long)__float_as_uint(t) << 32 | __float_as_uint(s), tag);
+    if (w >= 0)
+      st_word16(B.xst + tag % STR_ST_COPIES * B.words + w, (unsigned long long)__float_as_uint(t) << 32 | __float_as_uint(s), tag);
   };
   auto put_nu = [&](int k, float v, unsigned int tag) {
     const int w = __ldg(rexp + k);
