@@ -378,46 +378,53 @@ __device__ __forceinline__ bool red_sums(const RedArgs<T>& A, const RedTile<T>& 
   return !__syncthreads_or(fail);
 }
 
-// Start: r = b - A x (+ add) of the own rows and this block's share of the
-// group-0 rows (stored in A.rho), g, invd, x; sums |r_B|, r_B^2, |rho|, rho^2.
-template <typename T, int BS>
+// r = b - A x (+ add) of the own rows and this block's share of the group-0
+// rows (stored in A.rho), g; sums |r_B|, r_B^2, |rho|, rho^2 and, with NS = 5,
+// (d x)^2 over the rows of both.  first: the start of a solve, which also loads x and invd;
+// else A.x is what red_finish has stored.
+template <typename T, int BS, int NS>
 __device__ __forceinline__ bool red_start(const RedArgs<T>& A, const RedTile<T>& L, T* x, T* invd, T* g, T* r, T add,
-                                          double (&s4)[4], PhaseState& ph) {
+                                          double (&sum)[NS], PhaseState& ph, bool first = true) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, n = A.n, g1 = A.g1;
+  const bool zero = first && A.xzero;
   auto resid = [&](int row, T xr) {
-    T sum = T(0);
-    if (!A.xzero) {
+    T acc = T(0);
+    if (!zero) {
       const int kl = __ldg(A.nlo + row), ku = __ldg(A.nup + row);
       for (int s = 0; s < kl + ku; ++s) {
         const size_t e = (size_t)(s < kl ? s : A.KL + (s - kl)) * n + row;
-        sum = sum + __ldg(A.aoff + e) * A.x[__ldg(A.col + e)];
+        acc = acc + __ldg(A.aoff + e) * ldm(A.x + __ldg(A.col + e));
       }
-      sum = sum + __ldg(A.b + row) - __ldg(A.diag + row) * xr;
+      const T dx = __ldg(A.diag + row) * xr;
+      if constexpr (NS == 5) sum[4] += (double)dx * (double)dx;
+      acc = acc + __ldg(A.b + row) - dx;
     } else {
-      sum = __ldg(A.b + row);
+      acc = __ldg(A.b + row);
     }
-    return sum + add;
+    return acc + add;
   };
 #pragma unroll
-  for (int q = 0; q < 4; ++q) s4[q] = 0.0;
+  for (int q = 0; q < NS; ++q) sum[q] = 0.0;
   const int r1 = (int)((long long)g1 * (A.tile + 1) / A.nt);
   for (int row = (int)((long long)g1 * A.tile / A.nt) + (int)threadIdx.x; row < r1; row += BS) {
-    const T v = resid(row, A.xzero ? T(0) : A.x[row]);
+    const T v = resid(row, zero ? T(0) : ldm(A.x + row));
     A.rho[row] = v;
-    s4[2] += fabs((double)v);
-    s4[3] += (double)v * (double)v;
+    sum[2] += fabs((double)v);
+    sum[3] += (double)v * (double)v;
   }
   for (int j = wid; j < L.ns; j += (BS / 32)) {
     const int k = j * 32 + lane;
     if (k >= L.nb) continue;
     const int row = g1 + __ldg(A.trow + L.t0 + k);
-    const T xr = A.xzero ? T(0) : A.x[row];
+    const T xr = first ? (zero ? T(0) : A.x[row]) : x[k];
     const T v = resid(row, xr);
-    x[k] = xr;
     r[k] = v;
-    invd[k] = __ldg(A.invd + row);
-    s4[0] += fabs((double)v);
-    s4[1] += (double)v * (double)v;
+    if (first) {
+      x[k] = xr;
+      invd[k] = __ldg(A.invd + row);
+    }
+    sum[0] += fabs((double)v);
+    sum[1] += (double)v * (double)v;
   }
   grid_barrier(A, ph);  // A.rho written, A.x no longer read
   if (!ph.ok) return false;
@@ -580,15 +587,29 @@ __global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
 // step takes one reduction (vh_i.vh_i, vh_j.w, and vh_j.vh_i, which turn the
 // products with w into those of the modified Gram-Schmidt steps) instead of
 // 1 + i.  The norm that ends a step arrives with the next step's sums; a step
-// begun although the last one met the tolerance is dropped.  The next
-// residual is the combination of the vh_i that the Hessenberg relation gives.
+// begun although the last one met the tolerance is dropped.  The next cycle
+// starts from the combination of the vh_i that the Hessenberg relation gives,
+// until rounding may have taken that away from b - A x: then from b - A x
+// itself, as pgmres does at every restart.  A cycle adds about u |A||x| of
+// rounding to the difference (u the type's half unit, |A||x| taken as RED_DEV
+// |D x|, or of the first residual where that is larger); once the sum passes
+// RED_ETA of the residual it is computed anew and the sum starts over, the
+// rule of van der Vorst and Ye's residual replacement (SIAM J. Sci. Comput. 22,
+// 2000).  Near the attainable accuracy that is every cycle, so the stopping
+// test sees what it saw with a residual per restart; in FP64 down to about
+// 1e-11 of |D x| never.
+constexpr double RED_ETA = 1e-3, RED_DEV = 10.0;
+template <typename T> __device__ __forceinline__ constexpr double half_unit() { return sizeof(T) == 8 ? 1.1102230246251565e-16 : 5.9604644775390625e-08; }
+
 struct GmState {
   double h[4][3];         // h[j][i]: coefficients of step i, h[i+1][i] the norm
   double rt[4][3];        // the same, rotated
   double a[4], c[4];      // scale of vh_i, its group-0 multiple
   double rs[4], gc[3], gs[3], y[3], e[4];
   double ro, ro0, eps;
+  double dev, dx2;        // rounding since b - A x was formed, |D x|^2
   int i, inner, cyc, end, stop, nonfinite, converged;  // end: steps of the finished cycle
+  int renew;              // the next cycle starts from b - A x
 };
 
 // Closes step i (0-based) with the norm^2 of vh_{i+1}: scale, rotations, the
@@ -650,7 +671,8 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
     A.nt = A.ntiles = gridDim.x;
     A.tile = blockIdx.x;
     G.inner = G.cyc = G.stop = G.nonfinite = G.converged = 0;
-    G.ro = G.ro0 = G.eps = 0.0;
+    G.ro = G.ro0 = G.eps = G.dev = 0.0;
+    G.renew = 0;
     G.c[0] = 1.0;
   }
   __syncthreads();
@@ -670,21 +692,24 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
   };
   unsigned int tag = A.tag0;
   int buf = 0, cyc = 0;
-  double s4[4];
-  red_start<T, BS>(A, L, x, invd, g, v0, T(0), s4, ph);
-  bool ok = red_sums<T, BS, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
+  double s5[5];
+  red_start<T, BS>(A, L, x, invd, g, v0, T(0), s5, ph);
+  bool ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok);
   buf ^= 1;
-  const double rho2 = s_bc[3];
+  double rho2 = s_bc[3];
+  if (threadIdx.x == 0) G.dx2 = s_bc[4];
+  double dx2 = 0.0;  // of this thread's rows
+  bool stored = false;  // the result is in A.x
   while (ok && cyc < A.maxit) {
-    // step 1: w = A M^-1 vh_1 (into v1); vh_1.vh_1, vh_1.w
+    // step 1: w = A M^-1 vh_1 (into v1); vh_1.vh_1, vh_1.w, and |D x|^2 after the last cycle
     ok = red_apply<T, BS>(A, L, v0, g, invd, G.c[0], v1, tag++, 0);
-    double a2[2] = {0.0, 0.0};
+    double a3[3] = {0.0, 0.0, dx2};
     rows([&](int k) {
       const double p = v0[k];
-      a2[0] += p * p;
-      a2[1] += p * (double)v1[k];
+      a3[0] += p * p;
+      a3[1] += p * (double)v1[k];
     });
-    ok = red_sums<T, BS, 2>(A, L, a2, s_sum, s_bc, buf, tag++, !ok);
+    ok = red_sums<T, BS, 3>(A, L, a3, s_sum, s_bc, buf, tag++, !ok);
     buf ^= 1;
     if (!ok) break;
     if (threadIdx.x == 0) {
@@ -696,6 +721,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
       G.ro = G.rs[0] = ro;
       G.a[0] = 1.0 / (ro + SMALL);
       G.end = 0;
+      G.dx2 = fmax(G.dx2, 2.0 * s_bc[2]);  // (B rows: about half of them)
       const double h = G.a[0] * G.a[0] * (s_bc[1] + cc);
       G.h[0][0] = h;
       G.c[1] = G.a[0] * G.c[0] - h * G.a[0] * G.c[0];
@@ -792,6 +818,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
                       (m > 2 ? G.e[3] * G.c[3] : 0.0);
     const T y0 = (T)G.y[0], y1 = m > 1 ? (T)G.y[1] : T(0), y2 = m > 2 ? (T)G.y[2] : T(0), ct = (T)cy;
     const T e0 = (T)G.e[0], e1 = (T)G.e[1], e2 = m > 1 ? (T)G.e[2] : T(0), e3 = m > 2 ? (T)G.e[3] : T(0);
+    dx2 = 0.0;
     rows([&](int k) {
       const T p = v0[k], q = v1[k];
       T yv = y0 * p, rn = e0 * p + e1 * q;
@@ -806,7 +833,11 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
       }
       const unsigned short kd = L.kind[k];
       if (kd == RED_SIMPLE) {
-        x[k] = x[k] + invd[k] * (yv - ct * g[k]);
+        const T xk = x[k], di = invd[k];
+        const T xn = xk + di * (yv - ct * g[k]);
+        x[k] = xn;
+        const double dx = (double)xn / (double)di;
+        dx2 += dx * dx;
       } else {
         T z = y0 * L.os_z[kd];
         if (m > 1) z = z + y1 * L.os_z[L.nosp + kd];
@@ -817,11 +848,41 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
     });
     ++cyc;
     __syncthreads();  // G.c, G.y read
-    if (threadIdx.x == 0) G.c[0] = cn;
+    if (threadIdx.x == 0) {
+      G.c[0] = cn;
+      const bool fresh = G.dev == 0.0;
+      G.dev += half_unit<T>() * RED_DEV * fmax(sqrt(G.dx2), G.ro0);
+      G.renew = G.dev > RED_ETA * G.ro && !(G.stop && fresh) ? 1 : 0;
+    }
     __syncthreads();
-    if (G.stop) break;
+    if (!G.renew) {
+      if (G.stop) break;
+      continue;
+    }
+    if (cyc >= A.maxit && !G.stop) break;
+    red_finish<T, BS>(A, L, x, G.c[0], T(0), ph);
+    grid_barrier(A, ph);
+    if (ph.ok) red_start<T, BS>(A, L, x, invd, g, v0, T(0), s5, ph, false);
+    ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok);
+    buf ^= 1;
+    if (!ok) break;
+    rho2 = s_bc[3];
+    if (threadIdx.x == 0) {
+      G.c[0] = 1.0;
+      G.dev = 0.0;
+      G.dx2 = fmax(G.dx2, s_bc[4]);
+      if (G.stop) {  // met by the cycle's estimate: by the residual too?
+        G.ro = sqrt(s_bc[1] + rho2 + SMALL);
+        if (!(G.ro <= G.eps)) G.stop = 0;
+      }
+    }
+    __syncthreads();
+    if (G.stop) {
+      stored = true;
+      break;
+    }
   }
-  if (ok) {
+  if (ok && !stored) {
     ph.ok = true;
     red_finish<T, BS>(A, L, x, G.c[0], T(0), ph);
   }
