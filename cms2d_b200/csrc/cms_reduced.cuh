@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
   int it = 0, converged = 0, nonfinite = 0;
   while (ok && it < A.maxit) {
     ++it;
-    const double od = alf * bet0 + SMALL, omg = fast_div(bet * gam, od, fast_rcp(od));
+    const double omg = bet * gam / (alf * bet0 + SMALL);
     const T om = (T)omg, al = (T)alf;
     cp = cr + omg * (cp - alf * cu);
     rows([&](int k) { p[k] = r[k] + om * (p[k] - al * u[k]); });
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
     buf ^= 1;
     if (!ok) break;
     const double ukr0 = s_bc[0] + cu * rho2;
-    gam = fast_div(bet, ukr0, fast_rcp(ukr0));
+    gam = bet / ukr0;
     bet0 = bet;
     const T ga = (T)gam;
     cr = cr - gam * cu;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
     buf ^= 1;
     if (!ok) break;
     const double vr = s_bc[0] + cr * cr * rho2, vv = fmax(s_bc[1] + cr * cr * rho2, SMALL);
-    alf = fast_div(vr, vv, fast_rcp(vv));
+    alf = vr / vv;
     const T a2 = (T)alf;
     cr = cr - alf * cr;
     double s3[3] = {0.0, 0.0, 0.0};

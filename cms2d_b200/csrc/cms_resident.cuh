@@ -191,22 +191,6 @@ __device__ __forceinline__ bool collect_sums(double* bc, const ulonglong2* slots
   return fail;
 }
 
-// 1/d: the hardware's approximate reciprocal r (2^-20), refined by one cubic
-// step, with e = 1 - d r:  r (1 + e + e^2), error e^3.  A quotient n/d is n
-// times it, corrected by the remainder.  No branch, about a quarter of the
-// FP64 division's 430 cycles (measured); 0 and infinity give NaN, which the
-// callers' tests of the sums exclude.
-__device__ __forceinline__ double fast_rcp(double d) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-  const double e = fma(-d, r, 1.0);
-  return fma(r, fma(e, e, e), r);
-}
-__device__ __forceinline__ double fast_div(double n, double d, double rcp_d) {
-  const double q = n * rcp_d;
-  return fma(fma(-q, d, n), rcp_d, q);
-}
-
 // Scalars of one iteration, formed by one warp and read by the block, and the
 // recurrence's state, touched by that warp only (in shared memory: in
 // registers every thread would hold it).
@@ -247,20 +231,18 @@ __device__ __forceinline__ void resident_report(DevState* d, const ResState& st,
 
 // omg of an iteration, by every thread.
 __device__ __forceinline__ double resident_omega(const double* t) {
-  const double d = fmax(t[1], SMALL);
-  return fast_div(t[0], d, fast_rcp(d));
+  return t[0] / fmax(t[1], SMALL);
 }
 
 // The other scalars, from the sums of iteration it (as schur_body_sr).
 __device__ __forceinline__ void resident_scalars(const double* t, double omg, ResState& st, ResScal& sc, int it,
                                                  int maxit) {
-  const double alf = st.alf, rho = st.rho, d = fmax(t[1], SMALL);
-  const double rn = fast_rcp(t[0]), rrho = fast_rcp(rho);
+  const double alf = st.alf, rho = st.rho;
   const double rr = fmax(t[2] - 2.0 * omg * t[0] + omg * omg * t[1], 0.0);
   const double rho1 = t[3] - omg * t[4];
-  const double bet = (rho1 * rrho) * (alf * (d * rn));  // (rho1/rho) (alf/omg)
+  const double bet = (rho1 / rho) * (alf / omg);
   const double tau = (t[5] - omg * t[6]) + bet * (t[8] - omg * t[7]);
-  const double alf_n = fast_div(rho1, tau, fast_rcp(tau));
+  const double alf_n = rho1 / tau;
   const bool finite = isfinite(rr) && isfinite(omg) && isfinite(rho1);
   const bool save = finite && rr < st.best2;  // y += alf p + omg s is valid even at a breakdown below
   const double best2 = save ? rr : st.best2;

@@ -1,0 +1,28 @@
+"""The reduced FP64 BiCGStab and GMRES(3) at the ends of their ranges."""
+import numpy as np
+import pytest
+
+from cms2d_b200 import grid as G
+from cms2d_b200 import solver as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(s, system, scale=1.0, **kw):
+    acoef, ss, sp, phi = [a.copy() for a in system]
+    ss *= scale
+    info = s.solve(acoef, ss, sp, np.zeros_like(ss), phi, relax=1.0, **kw)
+    return info, phi
+
+
+@pytest.mark.parametrize("power", [400, 500, 506])
+def test_bicgstab_scales_with_its_right_hand_side(power):
+    """The recurrence is homogeneous and its added constants (1e-15) vanish in a right-hand side above 2^300, so scaling
+    by a power of two scales every number of the solve exactly: at 2^506 the squared sums are about 2^1022."""
+    g = G.cartesian_grid(33, 31)
+    system = G.random_system(g, seed=31)
+    s = S.Solver(g, tol=1e-8, norm=2, nsolv=3)
+    i0, p0 = _solve(s, system, 2.0 ** 300, nswp=300)
+    i1, p1 = _solve(s, system, 2.0 ** power, nswp=300)
+    assert i0["status"] == 0 and (i1["status"], i1["iters"]) == (0, i0["iters"]), (i0, i1)
+    np.testing.assert_array_equal(p1, p0 * 2.0 ** (power - 300))
