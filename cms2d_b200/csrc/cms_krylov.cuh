@@ -541,11 +541,12 @@ __global__ void __launch_bounds__(TPB) k_resid64(int n, int KL, GroupTab tab, co
 }
 
 // x64 += scale * d32 (refinement correction; scale undoes the normalisation),
-// unless the inner solve failed or there was nothing to correct
+// unless the inner solve failed, there was nothing to correct or the residual's
+// norm is not finite (the inner solve's right-hand side was then zero or NaN)
 __global__ void __launch_bounds__(TPB) k_ir_correct(int n, const float* __restrict__ d, double* __restrict__ x,
                                                     const DevState* st) {
   const double scale = st->s[S_IRSCALE];
-  if (st->nonfinite || st->bar.err || !(scale > 0.0)) return;
+  if (st->nonfinite || st->bar.err || !(scale > 0.0) || isinf(scale)) return;
   for (int i = blockIdx.x * TPB + threadIdx.x; i < n; i += gridDim.x * TPB) x[i] += scale * (double)d[i];
 }
 

@@ -1647,7 +1647,7 @@ static int refine_outcome(Solver* S, RefineState& R, bool& go) {
     R.nrm0 = R.prev = S->h_st->s[S_IRSCALE];
     R.rel = R.nrm0 > 0 ? 1.0 : 0.0;
     if (!std::isfinite(R.nrm0)) {
-      R.rel = R.nrm0;
+      R.rel = R.nrm0 / R.nrm0;
       R.info->status = CMS_NONFINITE;
       return CMS_OK;
     }

@@ -1,4 +1,4 @@
-"""The reduced FP64 BiCGStab and GMRES(3) at the ends of their ranges."""
+"""The reduced solves (FP64 BiCGStab, GMRES(3), refinement's inner solve) at the ends of their ranges."""
 import numpy as np
 import pytest
 
@@ -26,3 +26,17 @@ def test_bicgstab_scales_with_its_right_hand_side(power):
     i1, p1 = _solve(s, system, 2.0 ** power, nswp=300)
     assert i0["status"] == 0 and (i1["status"], i1["iters"]) == (0, i0["iters"]), (i0, i1)
     np.testing.assert_array_equal(p1, p0 * 2.0 ** (power - 300))
+
+
+@pytest.mark.parametrize("layout", [0, 5])
+@pytest.mark.parametrize("bad", [1e160, np.inf, np.nan])
+def test_refinement_of_a_residual_without_finite_norm_leaves_phi(layout, bad):
+    """A residual whose squares overflow, or that is not finite itself, is reported and phi comes back as it went in."""
+    g = G.cartesian_grid(33, 31)
+    acoef, ss, sp, phi = G.random_system(g, seed=31)
+    phi[: g.ncells] = np.random.default_rng(7).standard_normal(g.ncells)
+    ss[g.ncells // 2] = bad
+    s = S.Solver(g, precision="fp32_refine", tol=1e-8, norm=2, nsolv=3, reduced_layout=layout)
+    info, out = _solve(s, (acoef, ss, sp, phi), nswp=300)
+    assert info["status"] == 2, info  # CMS_NONFINITE
+    np.testing.assert_array_equal(out, phi)
