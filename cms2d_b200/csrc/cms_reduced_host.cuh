@@ -73,9 +73,9 @@ static int red_limit(Solver* S, size_t* limit) {
 // Tables of the reduced Krylov solves for the handle's pattern, built on first
 // use.  S->rd.state: 1 built, -1 the pattern or its size does not take them.
 static int red_tables(Solver* S) {
-  RedTables& R = S->rd;
-  if (R.state != 0) return CMS_OK;
-  R.state = -1;
+  if (S->rd.state != 0) return CMS_OK;
+  S->rd.state = -1;
+  RedTables R;
   const HostPattern& P = S->hp;
   if (P.G < 2 || P.G > GFLAT || schur_pattern(S) != CMS_OK || !S->sc_sym) return CMS_OK;
   size_t rs_limit = 0;
@@ -259,6 +259,7 @@ static int red_tables(Solver* S) {
   std::vector<int> hword(hrow.size());
   for (size_t k = 0; k < hrow.size(); ++k) hword[k] = word[hrow[k]];
   cudaStream_t s = S->stream;
+  AllocScope scope{S};
   auto put = [&](auto** d, const auto& h) -> int {
     CHK(S->alloc(d, h.size()));
     if (!h.empty()) CMS_CUDA(cudaMemcpyAsync(*d, h.data(), h.size() * sizeof(h[0]), cudaMemcpyHostToDevice, s));
@@ -295,6 +296,8 @@ static int red_tables(Solver* S) {
   R.nfwd = G - 2;
   R.limit = limit;
   R.state = 1;
+  S->rd = R;
+  scope.kept = true;
   return CMS_OK;
 }
 
@@ -376,8 +379,8 @@ static bool red_wanted(Solver* S, int nsolv, int maxit) {
 }
 
 // The solve of A x = b (W.b, W.x) by BiCGStab (nsolv 3) or GMRES(3) (nsolv 4)
-// on its own part of the factor.  Returns 1 when the launch is refused; does
-// not wait for the launch: the caller copies the state to the host and calls
+// on its own part of the factor.  Returns 1 when its buffers or the launch are
+// refused; does not wait for the launch: the caller copies the state to the host and calls
 // check_waits.
 template <typename T>
 static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, int norm, double tol, int xzero) {
@@ -389,9 +392,11 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   if (!B.coef) {
     P2* c = nullptr;
     T *cd = nullptr, *gv = nullptr;
-    CHK(S->alloc(&c, (size_t)R.pairs * 32));
-    CHK(S->alloc(&cd, (size_t)nB));
-    CHK(S->alloc(&gv, (size_t)RED_NV_BICG * R.npad));
+    AllocScope scope{S};
+    if (S->alloc(&c, (size_t)R.pairs * 32) || S->alloc(&cd, (size_t)nB) ||
+        S->alloc(&gv, (size_t)RED_NV_BICG * R.npad))
+      return 1;
+    scope.kept = true;
     B.coef = c;
     B.cdiag = cd;
     B.gvec = gv;

@@ -193,10 +193,25 @@ struct cms_solver {
   double prof_bytes[16] = {0};
   long long prof_count[16] = {0};
 
+  int refuse_from = 0, refuse_count = 0;  // allocations to be refused (cms_solver_alloc_selftest)
+
+  // A request that the device refuses leaves no error behind for the launches
+  // that follow: what asked for it may have a way to do without.
   template <typename P>
   int alloc(P** p, size_t count) {
-    size_t nb = std::max<size_t>(count, 1) * sizeof(P);
-    CMS_CUDA(cudaMalloc((void**)p, nb));
+    const size_t nb = std::max<size_t>(count, 1) * sizeof(P);
+    size_t ask = nb;
+    if (refuse_count > 0 && --refuse_from < 0) {
+      --refuse_count;
+      ask = (size_t)1 << 60;  // more than any device has
+    }
+    const cudaError_t e = cudaMalloc((void**)p, ask);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      *p = nullptr;
+      std::snprintf(g_last_error, sizeof(g_last_error), "allocation of %zu bytes: %s", ask, cudaGetErrorString(e));
+      return CMS_DEVICE_ERROR;
+    }
     CMS_CUDA(cudaMemsetAsync(*p, 0, nb, stream));
     allocs.push_back((void*)*p);
     bytes += nb;
@@ -207,6 +222,19 @@ struct cms_solver {
 namespace cms {
 
 using Solver = ::cms_solver;
+
+// Gives back the handle's allocations since its construction unless kept.
+struct AllocScope {
+  Solver* S;
+  size_t mark = S->allocs.size(), bytes = S->bytes;
+  bool kept = false;
+  ~AllocScope() {
+    if (kept) return;
+    cudaStreamSynchronize(S->stream);
+    for (; S->allocs.size() > mark; S->allocs.pop_back()) cudaFree(S->allocs.back());
+    S->bytes = bytes;
+  }
+};
 
 static inline int nblk(int rows) { return (rows + TPB - 1) / TPB; }
 // Grid of a row kernel: one row per thread up to 8 blocks of 256 threads per
@@ -1010,11 +1038,12 @@ static int schur_pattern(Solver* S) {
         ctr[e] = (int)((size_t)(hit - row) * nB + kk);
       }
     }
-    if (sym && (size_t)KC * nB <= (size_t)INT32_MAX) {
+    AllocScope scope{S};
+    sym = sym && (size_t)KC * nB <= (size_t)INT32_MAX;
+    if (sym) {
       CHK(S->alloc(&S->d_sctr, ctr.size()));
       CHK(S->alloc(&S->d_sst, (size_t)2 * n));
       CMS_CUDA(cudaMemcpyAsync(S->d_sctr, ctr.data(), ctr.size() * sizeof(int), cudaMemcpyHostToDevice, S->stream));
-      S->sc_sym = 1;
     }
     // where the products of the numeric kernels go (SchurMap)
     int KS = 1, K1 = 1;  // most couplings: of any row the kernels read, of a B row
@@ -1061,7 +1090,9 @@ static int schur_pattern(Solver* S) {
     S->sc_nnz = nnz;
     S->sc_e0b = e0b;
     S->sc_tiles = 0;
+    S->sc_sym = sym ? 1 : 0;
     S->sc_state = 1;
+    scope.kept = true;
   }
   return CMS_OK;
 }
@@ -2146,6 +2177,13 @@ const char* cms_gpu_version(void) { return "cmsgpu 0.1 (sm_100a)"; }
 int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int which) {
   if (!s || spin_limit == 0 || (which != 0 && which != 1)) return CMS_BAD_ARGUMENT;
   return cms::persist_wait_selftest(s, spin_limit, which);
+}
+
+int cms_solver_alloc_selftest(cms_solver* s, int first, int count) {
+  if (!s || first < 0 || count < 0) return CMS_BAD_ARGUMENT;
+  s->refuse_from = first;
+  s->refuse_count = count;
+  return CMS_OK;
 }
 
 int cms_solver_wait_selftest(cms_solver* s, unsigned int spin_limit) {

@@ -116,7 +116,10 @@ void cms_solver_default_opts(cms_solver_opts* opts);
 
 /* solv_init (source/solvers/solvers.f90:93-202) + indexm (sparse.f90:2-70):
  * copies the connectivity, builds the unknown ordering, the ELL sparsity
- * pattern and the sweep schedule, and allocates all device buffers.
+ * pattern and the sweep schedule, and allocates the device buffers.  Tables
+ * and buffers of the reduced and persistent forms are allocated by the first
+ * solve that takes them (for the FP64 reduced solves at 1M cells 0.19
+ * GB); one that is refused leaves the solve to a form without them.
  * iwet may be NULL (all wet). */
 int cms_solver_create(int ncells, int ncellsD, int nmaxfaces, const int* cell2cell, const int* ncface,
                       const int* iwet, const cms_solver_opts* opts, cms_solver** out);
@@ -515,6 +518,11 @@ int cms_solver_wait_selftest(cms_solver* s, unsigned int spin_limit);
  * after spin_limit polls.  Returns CMS_DEVICE_ERROR with the message (the
  * expected result); the handle stays usable. */
 int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int which);
+/* Failure-detection check of device allocations: after first more of the
+ * handle's, the next count are asked of the device at a size that it refuses.
+ * Tables and buffers of a faster form that are refused leave the solve to the
+ * form that does without them. */
+int cms_solver_alloc_selftest(cms_solver* s, int first, int count);
 
 /* Library version string. */
 const char* cms_gpu_version(void);
