@@ -331,10 +331,19 @@ static bool stream_choose(Solver* S) {
   RedTables& R = S->rd;
   size_t smem = 0;
   if (stream_vectors(R, R.limit, &smem) < 0) return false;
-  if (!S->st_coef &&
-      (S->alloc(&S->st_coef, (size_t)R.pairs * 32) || S->alloc(&S->st_vec, (size_t)SV_N * R.npad) ||
-       S->alloc(&S->st_xnu, R.words + 1)))
-    return false;
+  if (!S->st_coef) {
+    float2* coef = nullptr;
+    float* vec = nullptr;
+    unsigned long long* xnu = nullptr;
+    AllocScope scope{S};
+    if (S->alloc(&coef, (size_t)R.pairs * 32) || S->alloc(&vec, (size_t)SV_N * R.npad) ||
+        S->alloc(&xnu, R.words + 1))
+      return false;
+    scope.kept = true;
+    S->st_coef = coef;
+    S->st_vec = vec;
+    S->st_xnu = xnu;
+  }
   return true;
 }
 

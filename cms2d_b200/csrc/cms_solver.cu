@@ -196,7 +196,7 @@ struct cms_solver {
   int refuse_from = 0, refuse_count = 0;  // allocations to be refused (cms_solver_alloc_selftest)
 
   // A request that the device refuses leaves no error behind for the launches
-  // that follow: what asked for it may have a way to do without.
+  // that follow (what asked for it may have a way to do without), and *p as it was.
   template <typename P>
   int alloc(P** p, size_t count) {
     const size_t nb = std::max<size_t>(count, 1) * sizeof(P);
@@ -205,15 +205,16 @@ struct cms_solver {
       --refuse_count;
       ask = (size_t)1 << 60;  // more than any device has
     }
-    const cudaError_t e = cudaMalloc((void**)p, ask);
+    void* q = nullptr;
+    const cudaError_t e = cudaMalloc(&q, ask);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      *p = nullptr;
       std::snprintf(g_last_error, sizeof(g_last_error), "allocation of %zu bytes: %s", ask, cudaGetErrorString(e));
       return CMS_DEVICE_ERROR;
     }
-    CMS_CUDA(cudaMemsetAsync(*p, 0, nb, stream));
-    allocs.push_back((void*)*p);
+    allocs.push_back(q);
+    CMS_CUDA(cudaMemsetAsync(q, 0, nb, stream));
+    *p = (P*)q;
     bytes += nb;
     return CMS_OK;
   }
@@ -603,7 +604,8 @@ static int build_tiles(Solver* S, int nt) {
     if (S->alloc(&S->d_dep_idx, didx.size() + 1)) return 0;
     S->cap_dep = didx.size() + 1;
   }
-  if (!S->d_dep_ptr && (S->alloc(&S->d_dep_ptr, GRID_CAP + 1) || S->alloc(&S->d_progress, (size_t)GRID_CAP * kProgressStride))) return 0;
+  if (!S->d_dep_ptr && S->alloc(&S->d_dep_ptr, GRID_CAP + 1)) return 0;
+  if (!S->d_progress && S->alloc(&S->d_progress, (size_t)GRID_CAP * kProgressStride)) return 0;
   cudaStream_t s = S->stream;
   if (cudaMemcpyAsync(S->d_toff, toff.data(), toff.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
       cudaMemcpyAsync(S->d_dep_ptr, dptr.data(), dptr.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
@@ -1328,18 +1330,19 @@ static int resident_tables(Solver* S, int tiles) {
                                : (nb[tile_of[i]] + 31) / 32 * 32 + (int)(std::lower_bound(H.begin(), H.end(), c) - H.begin()));
     }
   }
-  if (!S->d_rlcol) {
-    CHK(S->alloc(&S->d_rlcol, lcol.size()));
-    CHK(S->alloc(&S->d_rexp, (size_t)nB));
-    CHK(S->alloc(&S->d_rtrow, (size_t)nB));
-    CHK(S->alloc(&S->d_rtptr, (size_t)GRID_CAP + 1));
-    CHK(S->alloc(&S->d_rhptr, (size_t)GRID_CAP + 1));
-    CHK(S->alloc(&S->d_rslptr, (size_t)GRID_CAP));
-    CHK(S->alloc(&S->d_rslots, (size_t)2 * (NSMAX * GRID_CAP + RES_TOT)));
-  }
+  auto want = [&](auto** d, size_t count) { return *d ? (int)CMS_OK : S->alloc(d, count); };  // once per handle
+  CHK(want(&S->d_rlcol, lcol.size()));
+  CHK(want(&S->d_rexp, (size_t)nB));
+  CHK(want(&S->d_rtrow, (size_t)nB));
+  CHK(want(&S->d_rtptr, (size_t)GRID_CAP + 1));
+  CHK(want(&S->d_rhptr, (size_t)GRID_CAP + 1));
+  CHK(want(&S->d_rslptr, (size_t)GRID_CAP));
+  CHK(want(&S->d_rslots, (size_t)2 * (NSMAX * GRID_CAP + RES_TOT)));
   if (words + 1 > S->rs_words) {
-    CHK(S->alloc(&S->d_rxst, words + 1));
+    ulonglong2* xst = nullptr;
+    CHK(S->alloc(&xst, words + 1));
     CHK(S->alloc(&S->d_rxnu, words + 1));
+    S->d_rxst = xst;
     S->rs_words = words + 1;
   }
   if (hrow.size() + 1 > S->cap_rhrow) {

@@ -17,6 +17,7 @@ pytestmark = pytest.mark.gpu
 FORMS = {
     "bicgstab": dict(nsolv=3),
     "gmres": dict(nsolv=4),
+    "refinement": dict(nsolv=3, precision="fp32_refine"),  # resident, then streamed, then the tiles' form
 }
 
 
