@@ -86,6 +86,11 @@ struct GmcPlan {  // launch of GMRES as one cluster: 0 not planned, 1 planned, -
   size_t smem = 0;
   const void* kern = nullptr;
 };
+struct TileTab {  // tables of a number of tiles of the persistent kernels
+  int tiles = 0;  // 0 not built, -1 not launchable
+  int *toff = nullptr, *dep_ptr = nullptr, *dep_idx = nullptr;
+  size_t cap_toff = 0, cap_dep = 0;  // capacities of toff / dep_idx
+};
 struct RedBuf {  // of one precision
   void *coef = nullptr, *cdiag = nullptr, *gvec = nullptr;
 };
@@ -118,12 +123,10 @@ struct cms_solver {
   int max_blocks = 0;
   // persistent BiCGStab: slots per group, tile tables, block partials [2][3][tiles]
   int *d_gkl = nullptr, *d_gku = nullptr;
-  int *d_toff = nullptr, *d_dep_ptr = nullptr, *d_dep_idx = nullptr;
   unsigned int* d_progress = nullptr;
   double* d_ppart = nullptr;
   bool tiles_set = false;  // their number was set by the caller
-  int ptiles = 0;  // tiles (= blocks) of the persistent kernel; 0 not built, -1 not launchable
-  size_t cap_toff = 0, cap_dep = 0;  // capacities of d_toff / d_dep_idx
+  cms::TileTab pt, ptw;  // of blocks of 256 threads and the reduced layouts; of one block of 1024 per SM (persist_wide)
   // reduced (Schur complement) inner solve of refinement (cms_schur.cuh):
   // Chat's pattern and values, 1/d and 1/s, neighbour tiles under Chat
   int sc_state = 0;  // 0 not built, 1 built, -1 not possible on this pattern
@@ -536,29 +539,30 @@ static int persist_capacity(int dev) {
                   GRID_CAP);
 }
 
-static int build_tiles(Solver* S, int nt);
+static int build_tiles(Solver* S, TileTab& tab, int nt);
+static int build_tiles(Solver* S, int nt) { return build_tiles(S, S->pt, nt); }
 
 // Tiles of the persistent kernel: one block per tile, every block resident,
 // at most one block per 256 rows.  Builds the tile tables on first use; 0
 // when the device cannot launch the kernel or a group does not keep natural
 // order.
 static int persist_tiles(Solver* S) {
-  if (S->ptiles != 0) return std::max(S->ptiles, 0);
+  if (S->pt.tiles != 0) return std::max(S->pt.tiles, 0);
   const int cap = persist_capacity(S->dev);
   if (cap <= 0) {
-    S->ptiles = -1;
+    S->pt.tiles = -1;
     return 0;
   }
   return build_tiles(S, std::min(cap, nblk(S->hp.n)));
 }
 
 // Tile tables for nt tiles (tile t = natural cells [t n / nt, (t+1) n / nt)).
-static int build_tiles(Solver* S, int nt) {
+static int build_tiles(Solver* S, TileTab& tab, int nt) {
   const HostPattern& P = S->hp;
   const int n = P.n;
   nt = std::max(1, std::min(std::min(nt, nblk(n)), GRID_CAP));
-  if (S->ptiles == nt) return nt;
-  S->ptiles = -1;
+  if (tab.tiles == nt) return nt;
+  tab.tiles = -1;
   // tile t = natural cells [tstart[t], tstart[t+1])
   std::vector<int> tstart(nt + 1), tile_nat(n);
   for (int t = 0; t <= nt; ++t) tstart[t] = (int)((long long)t * n / nt);
@@ -596,36 +600,39 @@ static int build_tiles(Solver* S, int nt) {
     dptr[t + 1] = (int)didx.size();
   }
   // buffers sized for the largest table built so far
-  if (toff.size() > S->cap_toff) {
-    if (S->alloc(&S->d_toff, toff.size())) return 0;
-    S->cap_toff = toff.size();
+  if (toff.size() > tab.cap_toff) {
+    if (S->alloc(&tab.toff, toff.size())) return 0;
+    tab.cap_toff = toff.size();
   }
-  if (didx.size() + 1 > S->cap_dep) {
-    if (S->alloc(&S->d_dep_idx, didx.size() + 1)) return 0;
-    S->cap_dep = didx.size() + 1;
+  if (didx.size() + 1 > tab.cap_dep) {
+    if (S->alloc(&tab.dep_idx, didx.size() + 1)) return 0;
+    tab.cap_dep = didx.size() + 1;
   }
-  if (!S->d_dep_ptr && S->alloc(&S->d_dep_ptr, GRID_CAP + 1)) return 0;
+  if (!tab.dep_ptr && S->alloc(&tab.dep_ptr, GRID_CAP + 1)) return 0;
   if (!S->d_progress && S->alloc(&S->d_progress, (size_t)GRID_CAP * kProgressStride)) return 0;
   cudaStream_t s = S->stream;
-  if (cudaMemcpyAsync(S->d_toff, toff.data(), toff.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
-      cudaMemcpyAsync(S->d_dep_ptr, dptr.data(), dptr.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
+  if (cudaMemcpyAsync(tab.toff, toff.data(), toff.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
+      cudaMemcpyAsync(tab.dep_ptr, dptr.data(), dptr.size() * sizeof(int), cudaMemcpyHostToDevice, s) ||
       (!didx.empty() &&
-       cudaMemcpyAsync(S->d_dep_idx, didx.data(), didx.size() * sizeof(int), cudaMemcpyHostToDevice, s)) ||
+       cudaMemcpyAsync(tab.dep_idx, didx.data(), didx.size() * sizeof(int), cudaMemcpyHostToDevice, s)) ||
       cudaStreamSynchronize(s))
     return 0;
-  S->ptiles = nt;
+  tab.tiles = nt;
   return nt;
 }
 
 // FP32 systems of more than 1024 rows per SM run as one block of 1024 threads
 // per SM instead of four of 256: a quarter of the blocks arrive at a barrier and
-// leave partial sums, and fewer tiles wait on each other (solve to 1e-5, same
-// bits: 152k cells 1728 -> 1533 us, 1M 2944 -> 2639 us telescoping; 1200 ->
-// 1008 us and 1919 -> 1798 us Cartesian).
-// Builds the tiles; not when cms_solver_set_tiles chose their number.
+// leave partial sums, and fewer tiles wait on each other (solve to 1e-5, the
+// same results on these systems: 152k cells 1728 -> 1533 us, 1M 2944 -> 2639 us
+// telescoping; 1200 -> 1008 us and 1919 -> 1798 us Cartesian).  Builds their
+// tables, which are their own: the tiles of a handle's other solves do not
+// depend on whether it has solved in FP32.  Not when cms_solver_set_tiles chose
+// the number of tiles.
 template <typename T>
 static bool persist_wide(Solver* S) {
-  if (sizeof(T) != 4 || S->tiles_set || S->hp.G > GFLAT) return false;
+  if (sizeof(T) != 4 || S->tiles_set || S->hp.G > GFLAT || S->ptw.tiles < 0) return false;
+  if (S->ptw.tiles > 0) return true;
   int nsm = 0, per = 0;
   if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, S->dev) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bicg_persistent<float, 1024>, 1024, 0) != cudaSuccess ||
@@ -633,7 +640,7 @@ static bool persist_wide(Solver* S) {
     cudaGetLastError();
     return false;
   }
-  return S->hp.n > nsm * 1024 && persist_tiles(S) > 0 && build_tiles(S, nsm) == nsm;
+  return S->hp.n > nsm * 1024 && persist_capacity(S->dev) > 0 && build_tiles(S, S->ptw, nsm) == nsm;
 }
 
 // Algorithmic bytes of one persistent launch (each array a phase touches
@@ -688,7 +695,7 @@ static PersistArgs<T> make_args(Solver* S, Mat<T>& A, Work<T>& W, int tiles, int
   }
   a.ntiles = tiles;
   a.gkl = S->d_gkl; a.gku = S->d_gku;
-  a.toff = S->d_toff; a.dep_ptr = S->d_dep_ptr; a.dep_idx = S->d_dep_idx; a.progress = S->d_progress;
+  a.toff = S->pt.toff; a.dep_ptr = S->pt.dep_ptr; a.dep_idx = S->pt.dep_idx; a.progress = S->d_progress;
   a.col = S->d_col; a.nlo = S->d_nlo; a.nup = S->d_nup;
   a.aoff = A.aoff; a.diag = A.diag; a.luoff = A.luoff; a.invd = A.invd;
   a.b = W.b; a.x = W.x; a.r = W.r; a.r0 = W.r0; a.p = W.p; a.u = W.u; a.v = W.v; a.z = W.z;
@@ -754,6 +761,9 @@ template <typename T>
 static int run_bicgstab_persistent(Solver* S, Mat<T>& A, Work<T>& W, int tiles, int maxit, int norm, double tol,
                                    int xzero, bool wide) {
   PersistArgs<T> a = make_args<T>(S, A, W, tiles, maxit, norm, tol, xzero);
+  if (wide) {
+    a.toff = S->ptw.toff; a.dep_ptr = S->ptw.dep_ptr; a.dep_idx = S->ptw.dep_idx;
+  }
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
   void* args[] = {&a};
@@ -765,7 +775,7 @@ static int run_bicgstab_persistent(Solver* S, Mat<T>& A, Work<T>& W, int tiles, 
   const cudaError_t e = cudaLaunchCooperativeKernel(kern, dim3(tiles), dim3(wide ? 1024 : TPB), args, 0, S->stream);
   if (e == cudaErrorCooperativeLaunchTooLarge) {
     cudaGetLastError();
-    S->ptiles = -1;
+    (wide ? S->ptw : S->pt).tiles = -1;
     return 1;
   }
   if (e != cudaSuccess) {
@@ -804,7 +814,7 @@ static int run_bicgstab(Solver* S, Mat<T>& A, Work<T>& W, int maxit, int norm, d
   if (do_factor) CHK(factor<T>(S, A));
   if (!S->opts.multi_kernel) {
     const bool wide = persist_wide<T>(S);
-    const int tiles = persist_tiles(S);
+    const int tiles = wide ? S->ptw.tiles : persist_tiles(S);
     if (tiles > 0) {
       const int rc = run_bicgstab_persistent<T>(S, A, W, tiles, maxit, norm, tol, xzero, wide);
       if (rc != 1) return rc;
@@ -1440,7 +1450,7 @@ static SchurArgs make_schur_args(Solver* S, int tiles, int maxit, double tol) {
   std::memset(&a, 0, sizeof(a));
   a.n = P.n; a.g1 = P.gstart[1]; a.nB = P.n - a.g1; a.KL = P.KL; a.G = P.G; a.KC = S->sc_KC;
   a.ntiles = tiles;
-  a.toff = S->d_toff; a.dep_ptr = S->d_sdep_ptr; a.dep_idx = S->d_sdep_idx; a.progress = S->d_progress;
+  a.toff = S->pt.toff; a.dep_ptr = S->d_sdep_ptr; a.dep_idx = S->d_sdep_idx; a.progress = S->d_progress;
   a.ccol = S->d_sccol; a.coff = S->d_scoff; a.ccnt = S->d_sccnt;
   a.col = S->d_col; a.nlo = S->d_nlo; a.nup = S->d_nup; a.aoff = S->A32.aoff; a.sinv = S->d_ssinv;
   a.b = S->W32.b; a.x = S->W32.x;
@@ -1757,7 +1767,7 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
                                                                                                             : SF_TILES;
   if (schur && form == SF_TILES) {  // the tiles of the reduced kernel's layout
     const int nt = schur_tiles(S, schur_layout_index(S));
-    schur = nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->ptiles) == CMS_OK;
+    schur = nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->pt.tiles) == CMS_OK;
   }
   const bool relax = !schur && mc_persist && S->opts.inner_relax && P.G > 2;
   struct RelaxScope {  // the flags describe A32's factor and its solves only while this solve runs
@@ -1788,7 +1798,7 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
     while (go) {
       refine_inner_limits(S->opts, R);
       KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
-      CHK(run_schur_bicgstab(S, S->ptiles, R.imax, R.itol, form));  // (the tiles of its layout)
+      CHK(run_schur_bicgstab(S, S->pt.tiles, R.imax, R.itol, form));  // (the tiles of its layout)
       CHK(refine_finish_step(S));
       CMS_CUDA(cudaStreamSynchronize(S->stream));
       CHK(refine_outcome(S, R, go));
