@@ -152,6 +152,7 @@ struct cms_solver {
   unsigned long long* d_rxnu = nullptr;
   size_t cap_rhrow = 0, cap_rsloff = 0;
   unsigned int rs_tag = 1;  // first tag not used by any launch so far
+  bool form_refused[3] = {false, false, false};  // launches of a SchurForm that the device refused
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   cms::RedTables rd;
   cms::RedBuf rd64, rd32;
@@ -197,6 +198,7 @@ struct cms_solver {
   long long prof_count[16] = {0};
 
   int refuse_from = 0, refuse_count = 0;  // allocations to be refused (cms_solver_alloc_selftest)
+  int refuse_launches = 0;                // reduced inner solves' launches to be refused (cms_solver_launch_selftest)
 
   // A request that the device refuses leaves no error behind for the launches
   // that follow (what asked for it may have a way to do without), and *p as it was.
@@ -1496,6 +1498,8 @@ static int resident_count(const Solver* S, int blocks) {
 #include "cms_reduced_host.cuh"
 namespace cms {
 
+enum SchurForm : int { SF_TILES = 0, SF_RESIDENT = 1, SF_STREAM = 2 };
+
 // The automatic layout of the reduced inner solve on a multicolour ordering:
 // the resident form where the system fits it.
 static bool resident_wanted(const Solver* S) {
@@ -1506,7 +1510,7 @@ static bool resident_wanted(const Solver* S) {
 
 // Whether the resident form runs; builds its tables when it does.
 static bool resident_choose(Solver* S) {
-  if (!resident_wanted(S)) return false;
+  if (!resident_wanted(S) || S->form_refused[SF_RESIDENT]) return false;
   size_t smem = 0;
   const int blocks = resident_blocks(S->dev, &smem);
   return blocks > 0 && resident_tables(S, resident_count(S, blocks)) == CMS_OK && S->rs_tiles > 0;
@@ -1545,8 +1549,9 @@ static int schur_tiles(Solver* S, int layout) {
 }
 
 // The reduced FP32 inner solve (W32.b -> W32.x) as one cooperative launch,
-// after k_ir_scale (which clears its barrier).  Does not wait for it.
-enum SchurForm : int { SF_TILES = 0, SF_RESIDENT = 1, SF_STREAM = 2 };
+// after k_ir_scale (which clears its barrier).  Does not wait for it.  Returns
+// 1 when the resident or streamed form needs more of the device than is free;
+// the handle's later solves do without it.
 static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, SchurForm form) {
   const bool resident = form == SF_RESIDENT;
   if (resident) tiles = S->rs_tiles;
@@ -1564,12 +1569,20 @@ static int run_schur_bicgstab(Solver* S, int tiles, int maxit, double tol, Schur
     CMS_CUDA(cudaMemsetAsync(S->d_progress, 0, sizeof(unsigned int) * tiles * kProgressStride, S->stream));
   void* args[] = {form == SF_STREAM ? (void*)&sa : (void*)&a};
   prof_begin(S);
+  const bool refuse = form != SF_TILES && S->refuse_launches > 0;
+  S->refuse_launches -= refuse;
   const cudaError_t e =
-      form == SF_STREAM ? cudaLaunchCooperativeKernel((const void*)k_schur_stream, dim3(tiles), dim3(STR_BS), args,
+      refuse ? cudaErrorCooperativeLaunchTooLarge
+      : form == SF_STREAM ? cudaLaunchCooperativeKernel((const void*)k_schur_stream, dim3(tiles), dim3(STR_BS), args,
                                                       ssmem, S->stream)
       : resident ? cudaLaunchCooperativeKernel(resident_kernel(S->rs_nr, false), dim3(tiles), dim3(RES_BS), args,
                                              S->rs_smem, S->stream)
                : cudaLaunchCooperativeKernel(L.single, dim3(tiles), dim3(L.bs), args, 0, S->stream);
+  if (e == cudaErrorCooperativeLaunchTooLarge && form != SF_TILES) {
+    cudaGetLastError();
+    S->form_refused[form] = true;
+    return 1;
+  }
   if (e != cudaSuccess) {
     std::snprintf(g_last_error, sizeof(g_last_error), "cooperative launch (reduced BiCGStab): %s",
                   cudaGetErrorString(e));
@@ -1761,14 +1774,15 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
                           persist_tiles(S) > 0;
   bool schur = mc_persist && S->opts.inner_relax == 2;
   // resident on the SMs, else streamed, else the tiles of the layout option
-  const SchurForm form = !schur ? SF_TILES
+  SchurForm form = !schur ? SF_TILES
                          : resident_choose(S) ? SF_RESIDENT
-                         : resident_wanted(S) && schur_pattern(S) == CMS_OK && S->sc_sym && stream_choose(S) ? SF_STREAM
+                         : resident_wanted(S) && schur_pattern(S) == CMS_OK && S->sc_sym && !S->form_refused[SF_STREAM] && stream_choose(S) ? SF_STREAM
                                                                                                             : SF_TILES;
-  if (schur && form == SF_TILES) {  // the tiles of the reduced kernel's layout
+  auto layout_tiles = [S] {  // the tiles of the reduced kernel's layout
     const int nt = schur_tiles(S, schur_layout_index(S));
-    schur = nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->pt.tiles) == CMS_OK;
-  }
+    return nt > 0 && build_tiles(S, nt) == nt && schur_neighbours(S, S->pt.tiles) == CMS_OK;
+  };
+  if (schur && form == SF_TILES) schur = layout_tiles();
   const bool relax = !schur && mc_persist && S->opts.inner_relax && P.G > 2;
   struct RelaxScope {  // the flags describe A32's factor and its solves only while this solve runs
     Solver* s;
@@ -1798,7 +1812,12 @@ static int run_refine(Solver* S, int nsolv, int maxit, double tol, cms_solve_inf
     while (go) {
       refine_inner_limits(S->opts, R);
       KLAUNCH(S, P_VEC, (double)n * 12, (k_ir_scale<<<gsz(n), TPB, 0, S->stream>>>(n, S->W64.r, S->W32.b, S->d_st)));
-      CHK(run_schur_bicgstab(S, S->pt.tiles, R.imax, R.itol, form));  // (the tiles of its layout)
+      const int rc = run_schur_bicgstab(S, S->pt.tiles, R.imax, R.itol, form);  // (the tiles of its layout)
+      if (rc == 1 && layout_tiles()) {
+        form = SF_TILES;
+        continue;
+      }
+      CHK(rc == 1 ? CMS_DEVICE_ERROR : rc);
       CHK(refine_finish_step(S));
       CMS_CUDA(cudaStreamSynchronize(S->stream));
       CHK(refine_outcome(S, R, go));
@@ -2190,6 +2209,12 @@ const char* cms_gpu_version(void) { return "cmsgpu 0.1 (sm_100a)"; }
 int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int which) {
   if (!s || spin_limit == 0 || (which != 0 && which != 1)) return CMS_BAD_ARGUMENT;
   return cms::persist_wait_selftest(s, spin_limit, which);
+}
+
+int cms_solver_launch_selftest(cms_solver* s, int count) {
+  if (!s || count < 0) return CMS_BAD_ARGUMENT;
+  s->refuse_launches = count;
+  return CMS_OK;
 }
 
 int cms_solver_alloc_selftest(cms_solver* s, int first, int count) {

@@ -523,6 +523,10 @@ int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int
  * Tables and buffers of a faster form that are refused leave the solve to the
  * form that does without them. */
 int cms_solver_alloc_selftest(cms_solver* s, int first, int count);
+/* The same for launches: the next count launches of the resident or streamed
+ * reduced inner solve are taken as refused for their size (a device with fewer
+ * free SMs than blocks); the refinement goes on in the tiles' form. */
+int cms_solver_launch_selftest(cms_solver* s, int count);
 
 /* Library version string. */
 const char* cms_gpu_version(void);

@@ -1,4 +1,4 @@
-"""A device allocation that is refused inside a solve: the solve goes on in the form that does without it, and later
+"""A device allocation or a launch that is refused inside a solve: the solve goes on in the form that does without it, and later
 solves of the handle are right too.  The refusal is a request larger than the device, made at every allocation of a
 first solve in turn (one refused, and that one and all that follow).
 
@@ -54,3 +54,20 @@ def test_refused_allocations(form):
             refused.append(held[0] != full)
             s.close()
         assert refused[0] and not refused[-1]  # every allocation of the solve had its turn
+
+
+@pytest.mark.parametrize("count", [1, 2])
+def test_refused_launch_of_the_resident_form(count):
+    """The refinement finishes in the tiles' form, and later solves of the handle keep to the forms that fit."""
+    g = G.solver_test_grid(4000)
+    system = G.random_system(g, seed=41)
+    kw = dict(tol=1e-9, norm=2, nsolv=3, precision="fp32_refine")
+    s = S.Solver(g, **kw)
+    _, ref = _solve(s, g, system)
+    s.close()
+    s = S.Solver(g, **kw)
+    _lib.lib().cms_solver_launch_selftest(s._h, count)  # 2: the streamed form's too
+    for _ in range(3):
+        info, x = _solve(s, g, system)
+        assert info["status"] == 0 and info["true_relres"] <= 1e-9, info
+        assert np.abs(x - ref).max() <= 2 * 1e-9 * 250 * np.sqrt(g.ncells) * np.abs(ref).max()
