@@ -82,6 +82,8 @@ def lib():
     L.cms_solver_launches.restype = C.c_longlong
     L.cms_solver_profile.argtypes = [vp, i]
     L.cms_solver_wait_selftest.argtypes = [vp, C.c_uint]
+    L.cms_solver_exchange_selftest.argtypes = [vp, C.c_uint]
+    L.cms_solver_tag_selftest.argtypes = [vp, C.c_uint]
     L.cms_solver_alloc_selftest.argtypes = [vp, i, i]
     L.cms_solver_launch_selftest.argtypes = [vp, i]
     L.cms_solver_refine_fallbacks.argtypes = [vp]

@@ -447,7 +447,7 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   a.col = S->d_col; a.nlo = S->d_nlo; a.nup = S->d_nup;
   a.gvec = (T*)B.gvec; a.npad = R.npad; a.nvs = nvs; a.mat_smem = mat;
   a.xw = R.xw; a.slots = R.slots; a.bar = &S->d_st->bar; a.st = S->d_st;
-  a.maxit = maxit; a.norm = norm; a.xzero = xzero; a.tol = tol; a.spin_limit = kSpinLimit;
+  a.maxit = maxit; a.norm = norm; a.xzero = xzero; a.tol = tol; a.spin_limit = S->spin_limit;
   CHK(red_tags(S, 8u * (unsigned int)maxit + 8u, &a.tag0));  // at most 8 per cycle, 5 per iteration
   CMS_CUDA(cudaMemsetAsync(&S->d_st->bar, 0, sizeof(GridBar), S->stream));
   void* args[] = {&a};

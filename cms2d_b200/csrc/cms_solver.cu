@@ -152,6 +152,8 @@ struct cms_solver {
   unsigned long long* d_rxnu = nullptr;
   size_t cap_rhrow = 0, cap_rsloff = 0;
   unsigned int rs_tag = 1;  // first tag not used by any launch so far
+  unsigned int spin_limit = cms::kSpinLimit;  // polls of an exchanged word (smaller in cms_solver_exchange_selftest)
+  int lost_words[2] = {-1, -1};               // halo words that it has redirected: resident, reduced Krylov
   bool form_refused[3] = {false, false, false};  // launches of a SchurForm that the device refused
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   cms::RedTables rd;
@@ -1461,7 +1463,7 @@ static SchurArgs make_schur_args(Solver* S, int tiles, int maxit, double tol) {
   a.s_t = reinterpret_cast<float2*>(S->d_sst);
   a.yb = S->W32.vv[4];
   a.part = S->d_ppart; a.bar = &S->d_st->bar; a.st = S->d_st;
-  a.maxit = maxit; a.tol = tol; a.spin_limit = kSpinLimit;
+  a.maxit = maxit; a.tol = tol; a.spin_limit = S->spin_limit;
   if (S->rs_tiles > 0) {
     a.lcol = S->d_rlcol; a.rexp = S->d_rexp; a.tptr = S->d_rtptr; a.trow = S->d_rtrow;
     a.hptr = S->d_rhptr; a.hrow = S->d_rhrow; a.slptr = S->d_rslptr; a.sloff = S->d_rsloff;
@@ -1514,6 +1516,31 @@ static bool resident_choose(Solver* S) {
   size_t smem = 0;
   const int blocks = resident_blocks(S->dev, &smem);
   return blocks > 0 && resident_tables(S, resident_count(S, blocks)) == CMS_OK && S->rs_tiles > 0;
+}
+
+// Makes the exchanges of the resident form and of the reduced Krylov solves
+// (with the streamed form) fail, or undoes it (spin_limit 0): the first halo
+// word becomes one that no tile stores, and a poll gives up after spin_limit.
+static int exchange_selftest(Solver* S, unsigned int spin_limit) {
+  int* word[2] = {S->rs_tiles > 0 ? S->d_rhrow : nullptr, S->rd.state == 1 ? S->rd.hword : nullptr};
+  const int spare[2] = {(int)S->rs_words - 1, (int)S->rd.words};
+  for (int k = 0; k < 2; ++k) {
+    if (!word[k]) continue;
+    int v = spare[k];
+    if (spin_limit > 0 && S->lost_words[k] < 0) {
+      CMS_CUDA(cudaMemcpyAsync(&S->lost_words[k], word[k], sizeof(int), cudaMemcpyDeviceToHost, S->stream));
+      CMS_CUDA(cudaStreamSynchronize(S->stream));
+    } else if (spin_limit == 0 && S->lost_words[k] >= 0) {
+      v = S->lost_words[k];
+      S->lost_words[k] = -1;
+    } else {
+      continue;
+    }
+    CMS_CUDA(cudaMemcpyAsync(word[k], &v, sizeof(int), cudaMemcpyHostToDevice, S->stream));
+    CMS_CUDA(cudaStreamSynchronize(S->stream));
+  }
+  S->spin_limit = spin_limit > 0 ? spin_limit : kSpinLimit;
+  return CMS_OK;
 }
 
 // Layout of the reduced kernel for this handle (cms_solver_opts.reduced_layout,
@@ -2209,6 +2236,17 @@ const char* cms_gpu_version(void) { return "cmsgpu 0.1 (sm_100a)"; }
 int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int which) {
   if (!s || spin_limit == 0 || (which != 0 && which != 1)) return CMS_BAD_ARGUMENT;
   return cms::persist_wait_selftest(s, spin_limit, which);
+}
+
+int cms_solver_exchange_selftest(cms_solver* s, unsigned int spin_limit) {
+  if (!s) return CMS_BAD_ARGUMENT;
+  return cms::exchange_selftest(s, spin_limit);
+}
+
+int cms_solver_tag_selftest(cms_solver* s, unsigned int tag) {
+  if (!s || tag < s->rs_tag || tag < s->rd.tag) return CMS_BAD_ARGUMENT;  // (a word may hold any earlier tag)
+  s->rs_tag = s->rd.tag = tag;
+  return CMS_OK;
 }
 
 int cms_solver_launch_selftest(cms_solver* s, int count) {

@@ -518,6 +518,16 @@ int cms_solver_wait_selftest(cms_solver* s, unsigned int spin_limit);
  * after spin_limit polls.  Returns CMS_DEVICE_ERROR with the message (the
  * expected result); the handle stays usable. */
 int cms_solver_persist_wait_selftest(cms_solver* s, unsigned int spin_limit, int which);
+/* The same for the exchanged words of the reduced solves (resident, streamed,
+ * reduced Krylov), in the kernels themselves: with spin_limit > 0 the first
+ * halo word of the tables that the handle has built is one that no tile
+ * stores, so that its next solve in such a form returns CMS_DEVICE_ERROR after
+ * spin_limit polls; 0 restores the words and the limit. */
+int cms_solver_exchange_selftest(cms_solver* s, unsigned int spin_limit);
+/* Sets the next tag of those words, which otherwise takes some 10^5 solves to
+ * come near the end of its 32 bits; tag not below the tags used so far
+ * (CMS_BAD_ARGUMENT otherwise). */
+int cms_solver_tag_selftest(cms_solver* s, unsigned int tag);
 /* Failure-detection check of device allocations: after first more of the
  * handle's, the next count are asked of the device at a size that it refuses.
  * Tables and buffers of a faster form that are refused leave the solve to the
