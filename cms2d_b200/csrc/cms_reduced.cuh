@@ -368,12 +368,14 @@ __device__ __forceinline__ bool red_apply(const RedArgs<T>& A, const RedTile<T>&
 }
 
 // Block sums, exchanged; the totals in bc for every thread.  False on a wait
-// that gave up.
+// that gave up.  all: values of every warp (the group-0 rows are dealt to all
+// threads), else of the warps that have slices of own rows.
 template <typename T, int BS, int NS>
 __device__ __forceinline__ bool red_sums(const RedArgs<T>& A, const RedTile<T>& L, double (&v)[NS],
-                                         double (*sm)[(BS / 32)], double* bc, int buf, unsigned int tag, bool fail) {
+                                         double (*sm)[(BS / 32)], double* bc, int buf, unsigned int tag, bool fail,
+                                         bool all = false) {
   ulonglong2* tot = A.slots + (size_t)2 * NSMAX * A.nt;
-  publish_sums<NS, (BS / 32)>(v, (int)(threadIdx.x >> 5) < L.ns, sm, A.slots, A.nt, A.tile, buf, tag);
+  publish_sums<NS, (BS / 32)>(v, all || (int)(threadIdx.x >> 5) < L.ns, sm, A.slots, A.nt, A.tile, buf, tag);
   fail |= collect_sums<NS, (BS / 32)>(bc, A.slots, tot, A.nt, A.tile, buf, tag, A.bar, A.spin_limit);
   return !__syncthreads_or(fail);
 }
@@ -504,7 +506,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_bicg(RedArgs<T> Ain) {
     p[k] = T(0);
     u[k] = T(0);
   });
-  bool ok = red_sums<T, BS, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok);
+  bool ok = red_sums<T, BS, 4>(A, L, s4, s_sum, s_bc, buf, tag++, !ph.ok, true);
   buf ^= 1;
   const double rho1 = s_bc[2], rho2 = s_bc[3];
   double bet = s_bc[1] + rho2;
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
   int buf = 0, cyc = 0;
   double s5[5];
   red_start<T, BS>(A, L, x, invd, g, v0, T(0), s5, ph);
-  bool ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok);
+  bool ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok, true);
   buf ^= 1;
   double rho2 = s_bc[3];
   if (threadIdx.x == 0) G.dx2 = s_bc[4];
@@ -863,7 +865,7 @@ __global__ void __launch_bounds__(BS, 1) k_red_gmres(RedArgs<T> Ain) {
     red_finish<T, BS>(A, L, x, G.c[0], T(0), ph);
     grid_barrier(A, ph);
     if (ph.ok) red_start<T, BS>(A, L, x, invd, g, v0, T(0), s5, ph, false);
-    ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok);
+    ok = red_sums<T, BS, 5>(A, L, s5, s_sum, s_bc, buf, tag++, !ph.ok, true);
     buf ^= 1;
     if (!ok) break;
     rho2 = s_bc[3];
