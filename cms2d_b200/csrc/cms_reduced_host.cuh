@@ -70,6 +70,41 @@ static int red_limit(Solver* S, size_t* limit) {
   return CMS_OK;
 }
 
+// What a tile of the reduced forms needs of shared memory at the least, as an
+// average over the tiles (own rows and own special rows only), so that a system
+// whose tiles cannot fit is left to the other forms without building the
+// tables first (9M cells: 1.7 s; the count takes 30 ms).
+static const RedRoom& red_room(Solver* S) {
+  RedRoom& M = S->rroom;
+  if (M.state != 0) return M;
+  M.state = -1;
+  const HostPattern& P = S->hp;
+  size_t rs_limit = 0;
+  const int blocks = resident_blocks(S->dev, &rs_limit);
+  if (P.G < 2 || P.G > GFLAT || blocks <= 0 || red_limit(S, &M.limit) != CMS_OK) return M;
+  const int n = P.n, g1 = P.gstart[1];
+  M.tiles = resident_count(S, blocks);
+  long long rows = 0, phases = 0, entries = 0;  // special rows, with their phases and the entries swept in these
+  for (int g = 1; g < P.G; ++g) {
+    for (int r = P.gstart[g]; r < P.gstart[g + 1]; ++r) {
+      int lo = 0;
+      for (int s = 0; s < P.nlo[r]; ++s) lo += P.col[(size_t)s * n + r] >= g1;
+      if (lo + P.nup[r] == 0) continue;
+      ++rows;
+      phases += g >= 2 ? 2 : 1;
+      entries += lo + P.nup[r];
+    }
+  }
+  auto krylov = [&](double T) {
+    return ((T + 2.0) * (n - g1) + (8.0 + T) * phases + (T + 2.0) * entries + (2.0 + 4.0 * T) * rows) / M.tiles;
+  };
+  M.krylov64 = krylov(sizeof(double));
+  M.krylov32 = krylov(sizeof(float));
+  M.stream = 2.0 * sizeof(float) * (n - g1) / M.tiles;
+  if (std::min(M.krylov64, M.stream) <= (double)M.limit) M.state = 1;  // (red_tables wants one of them to fit)
+  return M;
+}
+
 // Tables of the reduced Krylov solves for the handle's pattern, built on first
 // use.  S->rd.state: 1 built, -1 the pattern or its size does not take them.
 static int red_tables(Solver* S) {
@@ -327,6 +362,8 @@ static RedBuf& red_buf(Solver* S) {
 // us, 2.0M 87.3 / 27.4, 4.0M 156 / 66, 7.3M 280 / 150.  Bound by HBM at 4M and
 // above (about 70 % of the measured copy rate).
 static bool stream_choose(Solver* S) {
+  const RedRoom& M = red_room(S);
+  if (M.state != 1 || M.stream > (double)M.limit) return false;
   if (red_tables(S) != CMS_OK || S->rd.state != 1) return false;
   RedTables& R = S->rd;
   size_t smem = 0;
@@ -384,6 +421,8 @@ static bool red_wanted(Solver* S, int nsolv, int maxit) {
   if (S->opts.multi_kernel || S->opts.ordering != CMS_ORDER_MULTICOLOR || S->cur_relax || S->cur_fuse || maxit < 1 ||
       maxit > (1 << 26) || (nsolv == 3 && sizeof(T) == 4))
     return false;
+  const RedRoom& M = red_room(S);
+  if (M.state != 1 || (sizeof(T) == 8 ? M.krylov64 : M.krylov32) > (double)M.limit) return false;
   return red_tables(S) == CMS_OK && S->rd.state == 1;
 }
 
@@ -398,6 +437,10 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
   RedBuf& B = red_buf<T>(S);
   const int n = P.n, g1 = P.gstart[1], nB = n - g1;
   using P2 = typename Pair<T>::type;
+  const int nvec = nsolv == 3 ? RED_NV_BICG : RED_NV_GMRES;
+  int nvs = 0, mat = 0;
+  size_t smem = 0;
+  if (!red_plan<T>(R, nvec, R.limit, &nvs, &mat, &smem)) return 1;
   if (!B.coef) {
     P2* c = nullptr;
     T *cd = nullptr, *gv = nullptr;
@@ -410,10 +453,6 @@ static int run_reduced(Solver* S, Mat<T>& A, Work<T>& W, int nsolv, int maxit, i
     B.cdiag = cd;
     B.gvec = gv;
   }
-  const int nvec = nsolv == 3 ? RED_NV_BICG : RED_NV_GMRES;
-  int nvs = 0, mat = 0;
-  size_t smem = 0;
-  if (!red_plan<T>(R, nvec, R.limit, &nvs, &mat, &smem)) return 1;
   const double s = sizeof(T);
   int rc = CMS_OK;
   with_couplings(S->sc_KS, [&](auto ks) {

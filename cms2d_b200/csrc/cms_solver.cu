@@ -86,6 +86,11 @@ struct GmcPlan {  // launch of GMRES as one cluster: 0 not planned, 1 planned, -
   size_t smem = 0;
   const void* kern = nullptr;
 };
+struct RedRoom {  // shared memory a tile of the reduced forms needs at least, on average (cms_reduced_host.cuh)
+  int state = 0, tiles = 0;  // 0 not looked at, 1 known, -1 no tiles
+  size_t limit = 0;
+  double krylov64 = 0.0, krylov32 = 0.0, stream = 0.0;
+};
 struct TileTab {  // tables of a number of tiles of the persistent kernels
   int tiles = 0;  // 0 not built, -1 not launchable
   int *toff = nullptr, *dep_ptr = nullptr, *dep_idx = nullptr;
@@ -157,6 +162,7 @@ struct cms_solver {
   bool form_refused[3] = {false, false, false};  // launches of a SchurForm that the device refused
   long long reduced_fallbacks = 0;  // refinements finished on the exact factor after a bad inner correction
   cms::RedTables rd;
+  cms::RedRoom rroom;
   cms::RedBuf rd64, rd32;
   float2* st_coef = nullptr;  // streamed reduced solve: packed Chat, vectors, words of nu
   float* st_vec = nullptr;
@@ -1274,8 +1280,9 @@ static int resident_tables(Solver* S, int tiles) {
   const HostPattern& P = S->hp;
   const int g1 = P.gstart[1], nB = P.n - g1, KC = S->sc_KC;
   size_t limit = 0;
-  if (!S->sc_sym || tiles > resident_blocks(S->dev, &limit) || nB > (long long)tiles * RES_NRMAX * RES_BS)
-    return CMS_OK;
+  if (!S->sc_sym || tiles > resident_blocks(S->dev, &limit) || nB > (long long)tiles * RES_NRMAX * RES_BS ||
+      (0.5 * (sizeof(float2) + sizeof(ushort2)) * S->sc_nnz + 2.0 * sizeof(float) * nB) / tiles > (double)limit)
+    return CMS_OK;  // (the last: the tiles' average, without halo rows and padding)
   std::vector<int> ccol, tile_of, loc(nB), nb(tiles, 0), tptr(tiles + 1, 0), trow(nB);
   std::vector<signed char> cnt;
   CHK(schur_host_pattern(S, ccol, cnt));

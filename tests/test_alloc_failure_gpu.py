@@ -71,3 +71,16 @@ def test_refused_launch_of_the_resident_form(count):
         info, x = _solve(s, g, system)
         assert info["status"] == 0 and info["true_relres"] <= 1e-9, info
         assert np.abs(x - ref).max() <= 2 * 1e-9 * 250 * np.sqrt(g.ncells) * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("dtype", ["float64", "float32"])
+def test_no_tables_for_tiles_that_cannot_fit(dtype):
+    """Beyond about 8M cells a tile's gathered vector alone exceeds an SM's shared memory: nothing of the reduced forms is
+    built or allocated on the way to the form that runs."""
+    import torch
+    g = G.cartesian_grid(3000, 3001)
+    acoef, ss, sp, phi = [torch.from_numpy(a.astype(dtype)).cuda() for a in G.random_system(g, seed=5)]
+    s = S.Solver(g, nsolv=4)
+    before = s.device_bytes
+    info = s.solve(acoef, ss, sp, torch.zeros_like(ss), phi, relax=1.0, nswp=2)
+    assert info["iters"] == 2 and s.device_bytes == before
