@@ -631,14 +631,18 @@ static int build_tiles(Solver* S, TileTab& tab, int nt) {
   return nt;
 }
 
-// FP32 systems of more than 1024 rows per SM run as one block of 1024 threads
-// per SM instead of four of 256: a quarter of the blocks arrive at a barrier and
-// leave partial sums, and fewer tiles wait on each other (solve to 1e-5, the
-// same results on these systems: 152k cells 1728 -> 1533 us, 1M 2944 -> 2639 us
-// telescoping; 1200 -> 1008 us and 1919 -> 1798 us Cartesian).  Builds their
-// tables, which are their own: the tiles of a handle's other solves do not
-// depend on whether it has solved in FP32.  Not when cms_solver_set_tiles chose
-// the number of tiles.
+// FP32 systems of more than 1024 rows per SM, a row for every thread, run as one
+// block of 1024 threads per SM instead of four of 256: a quarter of the blocks
+// arrive at a barrier and leave partial sums, and fewer tiles wait on each
+// other.  Solve to 1e-5, 256 -> 1024 threads, the same iterations and results
+// on these systems: 160k cells 1728 -> 1606 us telescoping and 1200 -> 960
+// Cartesian, 1M 2944 -> 2639 and 1919 -> 1798.  Below the line, with 1024
+// threads there too: 148k 1666 -> 1556 and 1118 -> 958, 100k 1485 -> 1447 and
+// 972 -> 912, 75k 1460 -> 1445 and 961 -> 924, 40k 1495 -> 1580 and 921 -> 932:
+// the wide form gains from about 512 rows per SM on, a line at which it has not
+// been proven over all systems that it would change.  Builds its tables, which
+// are its own: the tiles of a handle's other solves do not depend on whether it
+// has solved in FP32.  Not when cms_solver_set_tiles chose the number of tiles.
 template <typename T>
 static bool persist_wide(Solver* S) {
   if (sizeof(T) != 4 || S->tiles_set || S->hp.G > GFLAT || S->ptw.tiles < 0) return false;
