@@ -13,7 +13,7 @@
 // split among the members in proportion to their unknowns, at least one
 // each.  When every member's tiles fit one SM each, the blocks are those of
 // the resident form of the reduced solves (six 10k-cell inlets, one step:
-// 146 ms with the streaming form, 83 ms resident); cms_ensemble_set_tiles
+// 146 ms with the form of cms_schur.cuh, 83 ms resident); cms_ensemble_set_tiles
 // picks the total (the autotuner in
 // cms2d_b200/ensemble.py times the candidates).
 #pragma once

@@ -18,7 +18,8 @@
 // and c, with the inner products of the full vectors (c c' rho.rho +
 // v_B.v'_B).  They are the same iterates as with triangular sweeps over the
 // whole matrix, up to rounding, on half the rows and with one gather per
-// operator application.  x_B collects M_S^-1 (v_B - c g); x_0 follows at the
+// operator application (GMRES looks at b - A x again where rounding has come
+// between it and the recurrence, see GmState).  x_B collects M_S^-1 (v_B - c g); x_0 follows at the
 // end from A's group-0 rows and the group-0 residual c rho.
 //
 // M_S is diagonal except at rows coupled to other B rows (telescoping

@@ -410,8 +410,8 @@ static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
 // k_bicg_persistent; so do refinement's inner solves with inner_relax 0 or 1.
 // Solve times, one B200 (per-phase kernels for GMRES, k_bicg_persistent for
 // BiCGStab / reduced form):
-//   GMRES(3) to 1e-3     20k cells 1.29 / 0.21 ms, 1M 4.39 / 0.75, 4M 10.7 / 2.8
-//   BiCGStab to 1e-6     100k cells 1.7 / 0.50 ms, 1M 4.9 / 1.13, 4M 14.0 / 5.3
+//   GMRES(3) to 1e-3     20k cells 1.29 / 0.21 ms, 1M 4.39 / 0.73, 4M 10.7 / 2.8
+//   BiCGStab to 1e-6     100k cells 1.7 / 0.49 ms, 1M 4.9 / 1.11, 4M 14.0 / 5.4
 // What bounds it: up to 250k cells the exchanges and sums (2 and 3 per
 // BiCGStab iteration, 3 and 4 per GMRES cycle), at 1M the coefficients read
 // from L2 (40 MB per application), at 4M HBM (160 MB per application and the

@@ -23,10 +23,10 @@
 //  * one warp forms the scalars of the recurrence while the others gather.
 //
 // Measured (one B200, kernel time per iteration, start and end of the launch
-// included, streaming form / this form): 1k cells 14.8 / 4.4 us, 30k 16.3 /
-// 4.6, 250k 16.9 / 6.4, 1M 28.8 / 15.0.  What bounds it: at 1M cells the
+// included, form of cms_schur.cuh / this form): 1k cells 14.7 / 4.4 us, 30k
+// 16.4 / 4.8, 250k 16.9 / 6.5, 1M 28.9 / 15.2.  What bounds it: at 1M cells the
 // shared-memory wavefronts of the two gathers (about 3000 cycles of 4400
-// each); at 30k cells the three exchanges through L2 (about 5000 of 8300
+// each); at 30k cells the three exchanges through L2 (about 5300 of 9000
 // cycles).
 //
 // Why a word is never overwritten too early.  nu of iteration i is replaced

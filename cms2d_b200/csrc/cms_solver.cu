@@ -1499,8 +1499,8 @@ static int resident_tags(Solver* S, int maxit, unsigned int* tag0) {
 }
 
 // Tiles of the resident form: one per SM, at least kResRows rows each (a
-// 30k-cell inlet-like system: 4.6 us per iteration with 128 rows, 5.2 with 256,
-// 5.3 with 512; fewer rows leave warps idle and add blocks to the sums).
+// 30k-cell inlet-like system: 4.6 us per iteration with 128 rows, 5.2 with 256
+// and 5.3 with 512 in one build, 4.8 with 128 now; fewer rows leave warps idle and add blocks to the sums).
 constexpr int kResRows = 128;
 static int resident_count(const Solver* S, int blocks) {
   const int nB = S->hp.n - S->hp.gstart[1];

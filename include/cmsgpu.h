@@ -282,7 +282,10 @@ int cms_pp_rhs_adjoint_dev_d(int ncells, int nmaxfaces, const int* cell2cell, co
                              const double* fintp, const double* grad_ss_pp, double* grad_acoef_u, double* grad_sp_u,
                              double* grad_hk, double* grad_u, double* grad_v, void* stream);
 /* Blocks (tiles) of the handle's persistent BiCGStab launch: 0 restores the
- * default (the device's resident capacity, at most one block per 256 rows);
+ * default (the device's resident capacity, at most one block per 256 rows; FP32
+ * systems of more than 1024 rows per SM one block of 1024 threads per SM).  The
+ * reduced forms (FP64 BiCGStab and GMRES on a multicolour ordering, refinement)
+ * have tiles of their own and do not follow it;
  * returns the count in use, or a negative CMS_* code. */
 int cms_solver_set_tiles(cms_solver* s, int tiles);
 /* The stream the handle runs on (a cudaStream_t). */
