@@ -413,9 +413,9 @@ static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
 //   GMRES(3) to 1e-3     20k cells 1.29 / 0.21 ms, 1M 4.39 / 0.73, 4M 10.7 / 2.8
 //   BiCGStab to 1e-6     100k cells 1.7 / 0.49 ms, 1M 4.9 / 1.11, 4M 14.0 / 5.4
 // What bounds it: up to 250k cells the exchanges and sums (2 and 3 per
-// BiCGStab iteration, 3 and 4 per GMRES cycle), at 1M the coefficients read
-// from L2 (40 MB per application), at 4M HBM (160 MB per application and the
-// vectors).
+// BiCGStab iteration, 3 and 4 per GMRES cycle); at 4M HBM (160 MB per
+// application and the vectors); at 1M not known: the coefficients come from L2
+// (40 MB per application), but at 2.2 TB/s, below what L2 gives.
 template <typename T>
 static bool red_wanted(Solver* S, int nsolv, int maxit) {
   if (S->opts.multi_kernel || S->opts.ordering != CMS_ORDER_MULTICOLOR || S->cur_relax || S->cur_fuse || maxit < 1 ||
