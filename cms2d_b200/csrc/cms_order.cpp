@@ -41,6 +41,15 @@ std::string build_pattern(int n, int nD, int nmf, const int* cell2cell, const in
       }
     }
   }
+  P.symmetric = true;
+  for (int i = 0; i < n && P.symmetric; ++i) {
+    for (int k = 0; k < nmf; ++k) {
+      const int j = adj[(size_t)i * nmf + k];
+      if (j < 0) continue;
+      const int* back = &adj[(size_t)j * nmf];
+      P.symmetric = P.symmetric && std::find(back, back + nmf, i) != back + nmf;
+    }
+  }
   // groups
   std::vector<int> grp(n, 0);
   if (ordering == 0) {

@@ -13,6 +13,7 @@ struct HostPattern {
   int nD = 0;         // active + dummy cells
   int nmf = 0;        // nmaxfaces
   int G = 0;          // groups (colours or levels)
+  bool symmetric = true;  // every coupling has its counterpart, so the groups of the multicolour ordering are independent
   int KL = 0, KU = 0; // lower / upper ELL slots (slot s < KL lower, KL <= s < KL+KU upper)
   std::vector<int> gstart;   // [G+1] device-row range of each group
   std::vector<int> gkl, gku; // [G] max lower / upper entries of rows in the group

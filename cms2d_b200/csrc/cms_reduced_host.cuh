@@ -81,7 +81,7 @@ static const RedRoom& red_room(Solver* S) {
   const HostPattern& P = S->hp;
   size_t rs_limit = 0;
   const int blocks = resident_blocks(S->dev, &rs_limit);
-  if (P.G < 2 || P.G > GFLAT || blocks <= 0 || red_limit(S, &M.limit) != CMS_OK) return M;
+  if (!P.symmetric || P.G < 2 || P.G > GFLAT || blocks <= 0 || red_limit(S, &M.limit) != CMS_OK) return M;
   const int n = P.n, g1 = P.gstart[1];
   M.tiles = resident_count(S, blocks);
   long long rows = 0, phases = 0, entries = 0;  // special rows, with their phases and the entries swept in these
@@ -402,7 +402,9 @@ static int stream_args(Solver* S, int maxit, StreamArgs* a, size_t* smem) {
   return red_tags(S, (unsigned int)maxit + 2u, &a->S.tag0);
 }
 
-// Whether a solve runs in reduced form: a multicolour ordering whose tiles'
+// Whether a solve runs in reduced form: a multicolour ordering of a symmetric
+// pattern (a cell that is not its neighbour's neighbour may share its group, and
+// group 0 is then not independent) whose tiles'
 // gathered vector fits an SM's shared memory (red_tables; about 8M cells in
 // FP64), on the exact factor.  BiCGStab only in FP64: in FP32 its recurrence
 // turns rounding into a different iteration count in one solve of seven

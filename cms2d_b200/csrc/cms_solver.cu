@@ -873,7 +873,7 @@ static int run_gmres_cluster(Solver* S, Mat<T>& A, Work<T>& W, int maxit, double
   cfg.numAttrs = 1;
   if (L.state == 0) {  // the launch's shape, once per handle and precision
     L.state = -1;
-    if (P.n > GMC_ROWS || P.G > 8 || P.G < 1 || S->tab.ng != P.G || S->tab.blk[S->tab.ng] > GMC_PART ||
+    if (!P.symmetric || P.n > GMC_ROWS || P.G > 8 || P.G < 1 || S->tab.ng != P.G || S->tab.blk[S->tab.ng] > GMC_PART ||
         P.gkl[0] != 0)
       return 1;
     int nslot = 0;
@@ -1517,7 +1517,7 @@ enum SchurForm : int { SF_TILES = 0, SF_RESIDENT = 1, SF_STREAM = 2 };
 // the resident form where the system fits it.
 static bool resident_wanted(const Solver* S) {
   const int lay = S->opts.reduced_layout;
-  return !(lay >= 1 && lay <= kSchurLayouts) && S->opts.inner_relax == 2 &&
+  return S->hp.symmetric && !(lay >= 1 && lay <= kSchurLayouts) && S->opts.inner_relax == 2 &&
          S->opts.ordering == CMS_ORDER_MULTICOLOR && S->hp.G >= 2;
 }
 
