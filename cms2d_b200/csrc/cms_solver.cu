@@ -648,13 +648,17 @@ static bool persist_wide(Solver* S) {
   if (sizeof(T) != 4 || S->tiles_set || S->hp.G > GFLAT || S->ptw.tiles < 0) return false;
   if (S->ptw.tiles > 0) return true;
   int nsm = 0, per = 0;
-  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, S->dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bicg_persistent<float, 1024>, 1024, 0) != cudaSuccess ||
+  if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, S->dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (S->hp.n <= nsm * 1024) return false;  // (before the occupancy query, which every smaller solve would pay for)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bicg_persistent<float, 1024>, 1024, 0) != cudaSuccess ||
       per < 1) {
     cudaGetLastError();
     return false;
   }
-  return S->hp.n > nsm * 1024 && persist_capacity(S->dev) > 0 && build_tiles(S, S->ptw, nsm) == nsm;
+  return persist_capacity(S->dev) > 0 && build_tiles(S, S->ptw, nsm) == nsm;
 }
 
 // Algorithmic bytes of one persistent launch (each array a phase touches
